@@ -37,8 +37,7 @@ Status bad(int code, const std::string &m) {
 }
 
 // Default shape: the single problem's default kernel and rule.  FP64: the lane kernel (warps = 0) with 16-wide
-// segments at DG degree 2, 8-wide at degree 1 for up to 24 ordinates per quadrant, else the narrowest segment
-// with the best lane use.  FP32_REFINED: the modal kernel, narrowest best segment, its default warps.
+// segments at DG degree 2, else the narrowest segment with the best lane use.  FP32_REFINED: the modal kernel, narrowest best segment, its default warps.
 void default_shape(int P, int precision, int qmax, int *seg, int *wn) {
     const bool lane = precision == IDC_PREC_FP64;
     double best = -1.0;
@@ -51,7 +50,7 @@ void default_shape(int P, int precision, int qmax, int *seg, int *wn) {
             *seg = cand;
         }
     }
-    if (lane && (P == 3 || (P == 2 && qmax <= 24))) *seg = P == 3 ? 16 : 8;
+    if (lane && P == 3) *seg = 16;
     *wn = lane ? 0 : sweep_modal_default_wn(P);
 }
 
@@ -101,9 +100,22 @@ Status Batch::build_group(Group &g, int precision) {
     if (lane && (precision != IDC_PREC_FP64 || !sweep_lane_supports(c0.P, 0, g.seg)))
         return bad(IDC_ERR_UNSUPPORTED, "batched lane sweeps: FP64, seg 4, 8 or 16");
     if (!lane) g.wn = sweep_modal_fit_wn(c0.P, precision, g.wn, g.G, g.seg);
-    const int seg = g.seg, wn = g.wn, rw = 32 / seg, rows_cta = lane ? rw : wn * rw;
+    const int seg = g.seg, rw = 32 / seg;
+    if (lane) {
+        g.lane_wn = sweep_lane_warps(c0.P, seg, false, c0.num_sms, [&](int w) {
+            int64_t blocks = 0;   // over all members
+            for (int p : g.members) {
+                const Context &c = *members[p];
+                for (int k = 0; k < 4; ++k)
+                    blocks += ((c.quad[k + 1] - c.quad[k] + seg - 1) / seg) * ((c.ny + w * rw - 1) / (w * rw));
+            }
+            return blocks;
+        });
+    }
+    const int wn = lane ? g.lane_wn : g.wn, rows_cta = wn * rw;
     std::vector<std::vector<SweepItem>> per(g.members.size());
     std::vector<int> nrb(g.members.size()), ipr(g.members.size());
+    g.slot_begin.assign(g.members.size(), {});
     for (size_t m = 0; m < g.members.size(); ++m) {
         const Context &c = *members[g.members[m]];
         // chunks of each quadrant (near-equal, at most seg ordinates)
@@ -122,6 +134,8 @@ Status Batch::build_group(Group &g, int precision) {
             }
         }
         ipr[m] = (int)qk.size();
+        for (int k = 0; k < 5; ++k)   // each quadrant's chunks, the partial-moment slots
+            g.slot_begin[m][k] = (int)(std::lower_bound(qk.begin(), qk.end(), k) - qk.begin());
         nrb[m] = (int)((c.ny + rows_cta - 1) / rows_cta);
         for (int rb = 0; rb < nrb[m]; ++rb)
             for (int s = 0; s < ipr[m]; ++s)
@@ -160,11 +174,11 @@ Status Batch::build_group(Group &g, int precision) {
         IDC_TRY_CUDA(cudaMalloc(&g.inflow[m], sizeof(double) * (size_t)(c.nx + c.ny) * c.nq * c.P));
     }
     int per_sm = 0;
-    if (lane) {   // shared memory fixed per kernel instance (set by the launcher); one item per warp at a time
+    if (lane) {   // shared memory set by the launcher
         g.smem = 0;
-        IDC_TRY_CUDA(sweep_lane_batched_occupancy(c0.P, seg, &per_sm));
+        IDC_TRY_CUDA(sweep_lane_batched_occupancy(c0.P, seg, wn, &per_sm));
         if (per_sm < 1) return bad(IDC_ERR_UNSUPPORTED, "batched sweep kernel does not fit on an SM");
-        g.grid = std::min((g.n_items + sweep_lane_warps() - 1) / sweep_lane_warps(), per_sm * c0.num_sms);
+        g.grid = std::min(g.n_items, per_sm * c0.num_sms);
     } else {
         g.smem = sweep_modal_smem_bytes(c0.P, precision, wn, g.G, seg);
         IDC_TRY_CUDA(sweep_modal_occupancy(c0.P, precision, seg, sweep_modal_threads(c0.P, wn), g.smem, &per_sm));
@@ -177,7 +191,7 @@ Status Batch::build_group(Group &g, int precision) {
 }
 
 Status Batch::launch_group(Group &g, const double *const *srcs, double *const *outs, const double *const *phi_sc,
-                           double scale, double *const *phis, double dt, const std::vector<char> *active) {
+                           double scale, double *const *phis, double dt, const std::vector<char> *active, bool peierls) {
     Context &c0 = *members[g.members[0]];
     cudaStream_t st = stream();
     std::vector<SweepArgs> table(g.members.size());
@@ -190,7 +204,14 @@ Status Batch::launch_group(Group &g, const double *const *srcs, double *const *o
         a.out = outs ? outs[p] : nullptr;
         a.sigma_t = c.d_sigma_t;
         a.sigma_s = nullptr;   // the modal kernel's fused source takes ready scattering moments
-        a.phi_scatter = phi_sc ? phi_sc[p] : nullptr;
+        if (g.wn == 0 && peierls) {   // moments-only: the vectors themselves, the modal sources formed on the device
+            a.sigma_s = c.d_sigma_s;
+            a.phi_scatter = phi_sc[p];
+            a.modal_src = c.d_msrc;
+            std::copy(g.slot_begin[m].begin(), g.slot_begin[m].end(), a.slot_begin);
+        } else {
+            (g.wn == 0 ? a.cell_rec : a.phi_scatter) = phi_sc ? phi_sc[p] : nullptr;
+        }
         a.scatter_scale = scale;
         a.xi = c.d_xi;
         a.eta = c.d_eta;
@@ -206,8 +227,8 @@ Status Batch::launch_group(Group &g, const double *const *srcs, double *const *o
         a.G = g.G;
         a.n_refine = 1;
         a.seg = g.seg;
-        a.wn = g.wn;
-        a.R = (g.wn == 0 ? 1 : g.wn) * (32 / g.seg);
+        a.wn = g.wn == 0 ? g.lane_wn : g.wn;
+        a.R = a.wn * (32 / g.seg);
         a.trace = g.trace[m];
         a.trace_stride = (size_t)c.nx * g.G * c.P;
         a.next_item = g.d_sync;
@@ -225,6 +246,8 @@ Status Batch::launch_group(Group &g, const double *const *srcs, double *const *o
             a.src = nullptr;
             a.out = nullptr;
             a.phi_scatter = nullptr;
+            a.cell_rec = nullptr;
+            a.modal_src = nullptr;
             a.phi = nullptr;
             a.phi_part = nullptr;
             a.inflow = nullptr;
@@ -251,16 +274,16 @@ Status Batch::launch_group(Group &g, const double *const *srcs, double *const *o
                                             true, false, st));
     IDC_TRY_CUDA(cudaMemsetAsync(g.d_sync, 0, sizeof(int), st));
     if (g.wn == 0)
-        IDC_TRY_CUDA(launch_sweep_lane_batched(c0.P, launch, g.d_table, g.grid, st));
+        IDC_TRY_CUDA(launch_sweep_lane_batched(c0.P, launch, g.d_table, (int)table.size(), peierls, g.grid, st));
     else
         IDC_TRY_CUDA(launch_sweep_modal_batched(c0.P, g.precision, launch, g.d_table, g.grid, g.smem, st));
-    if (any_phi)
+    if (any_phi && !(g.wn == 0 && peierls))
         IDC_TRY_CUDA(launch_batched_helpers(c0.P, false, g.d_table, (int)table.size(), false, true, st));
     return Status::ok();
 }
 
 Status Batch::sweep(const double *const *srcs, double *const *outs, const double *const *phi_sc, double scale,
-                    double *const *phis, double dt, int precision, const std::vector<char> *active) {
+                    double *const *phis, double dt, int precision, const std::vector<char> *active, bool peierls) {
     if (members.empty()) return bad(IDC_ERR_STATE, "empty batch");
     if (precision != IDC_PREC_FP64 && precision != IDC_PREC_FP32_REFINED)
         return bad(IDC_ERR_UNSUPPORTED, "batched sweeps run in FP64 or refined precision");
@@ -290,7 +313,7 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
         for (auto &g : groups) IDC_TRY(build_group(g, precision));
     }
     IDC_TRY_CUDA(cudaEventRecord(c0.ev0, c0.stream));
-    for (auto &g : groups) IDC_TRY(launch_group(g, srcs, outs, phi_sc, scale, phis, dt, active));
+    for (auto &g : groups) IDC_TRY(launch_group(g, srcs, outs, phi_sc, scale, phis, dt, active, peierls));
     IDC_TRY_CUDA(cudaEventRecord(c0.ev1, c0.stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(c0.stream));
     for (auto &g : groups) {
@@ -340,7 +363,7 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
         double beta = 0, resid = 0;
         int j = 0;
         int64_t its = 0;
-        bool done = false, converged = false, restart_pending = false;
+        bool done = false, converged = false, restart_pending = false, records = false;
         double *in = nullptr, *out = nullptr;
         double *Vc(int k) const { return V + (size_t)k * n; }
         double *Zc(int k) const { return V + (size_t)(m + 1 + k) * n; }   // flexible GMRES: Z after V_0 .. V_m
@@ -353,6 +376,13 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
     } free_err{d_err};
     IDC_TRY_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * M, st));
     std::vector<State> S(M);
+    auto scatter = [&](State &z, const double *phi) -> Status {
+        if (z.records)
+            IDC_TRY_CUDA(launch_cell_records(z.c->dims(), z.c->d_sigma_t, z.c->d_sigma_s, phi, z.scat, st));
+        else
+            IDC_TRY_CUDA(launch_scatter_moments(z.c->dims(), z.c->d_sigma_s, phi, z.scat, st));
+        return Status::ok();
+    };
     for (size_t p = 0; p < M; ++p) {
         Context &c = *members[p];
         State &z = S[p];
@@ -375,7 +405,31 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
         z.b = c.phi_buf(3);
         z.x = c.phi_buf(4);
         z.tmp = c.phi_buf(5);
-        z.scat = c.phi_buf(6);
+        // the scattering term of a batched sweep: the lane kernel's cell records, else the moments alone
+        int sg = 0, wn = 0;
+        get_shape(c.P, precision, &sg, &wn);
+        z.records = wn == 0;
+        if (z.records) {
+            const size_t need_rec = c.sig_len() * cell_record_doubles(c.P);
+            if (c.scat_len < need_rec) {
+                cudaFree(c.d_scat);
+                c.d_scat = nullptr;
+                c.scat_len = 0;
+                IDC_TRY_CUDA(cudaMalloc(&c.d_scat, sizeof(double) * need_rec));
+                c.scat_len = need_rec;
+            }
+        }
+        z.scat = z.records ? c.d_scat : c.phi_buf(6);
+        if (z.records) {   // the Krylov sweeps' modal sources
+            const size_t need_src = c.sig_len() * 4 * cell_record_doubles(c.P);
+            if (c.msrc_len < need_src) {
+                cudaFree(c.d_msrc);
+                c.d_msrc = nullptr;
+                c.msrc_len = 0;
+                IDC_TRY_CUDA(cudaMalloc(&c.d_msrc, sizeof(double) * need_src));
+                c.msrc_len = need_src;
+            }
+        }
         z.H.assign((size_t)(m + 1) * m, 0.0);
         z.cs.assign(m, 0.0);
         z.sn.assign(m, 0.0);
@@ -437,41 +491,43 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
             State &z = S[p];
             if (z.done) continue;
             Context &c = *z.c;
-            if (z.restart_pending) {
-                z.in = z.x;
-                z.out = z.Vc(0);
-            } else {
-                if (z.dsa) {
-                    IDC_TRY_CUDA(dsa_precondition(c.dims(), c.d_sigma_s, z.Vc(z.j), z.Zc(z.j), c.dsa_steps, c.d_dsa_ws,
-                                                  false, c.num_sms, d_err + p, c.spin_limit, st));
-                    z.in = z.Zc(z.j);
-                } else {
-                    z.in = z.Vc(z.j);
-                }
-                z.out = z.Vc(z.j + 1);
-            }
-            IDC_TRY_CUDA(launch_scatter_moments(c.dims(), c.d_sigma_s, z.in, z.scat, st));
+            z.in = z.restart_pending ? z.x : z.dsa ? z.Zc(z.j) : z.Vc(z.j);
+            z.out = z.restart_pending ? z.Vc(0) : z.Vc(z.j + 1);
+            if (!z.restart_pending && z.dsa)
+                IDC_TRY_CUDA(dsa_precondition(c.dims(), c.d_sigma_s, z.Vc(z.j), z.Zc(z.j), c.dsa_steps, c.d_dsa_ws, false,
+                                              c.num_sms, d_err + p, c.spin_limit, st));
         }
-        IDC_TRY(sweep(nullptr, nullptr, scats.data(), 1.0, tmps.data(), dt, precision, &active));
+        // lane-kernel members: out = in - P L^{-1} S in straight from the vectors; modal ones: P L^{-1} of S in, formed here
+        for (size_t p = 0; p < M; ++p) {
+            State &z = S[p];
+            if (z.done) continue;
+            scats[p] = z.records ? z.in : z.scat;
+            tmps[p] = z.records ? z.out : z.tmp;
+            if (!z.records) IDC_TRY(scatter(z, z.in));
+        }
+        IDC_TRY(sweep(nullptr, nullptr, scats.data(), 1.0, tmps.data(), dt, precision, &active, true));
         for (size_t p = 0; p < M; ++p) {
             State &z = S[p];
             if (z.done) continue;
             Context &c = *z.c;
             const size_t n = z.n;
-            IDC_TRY_CUDA(launch_axpby(1.0, z.in, 0.0, z.out, n, st));     // A in = in - P L^{-1} S in
-            IDC_TRY_CUDA(launch_axpby(-1.0, z.tmp, 1.0, z.out, n, st));
-            double *ds = c.d_small, *scratch = c.d_small + 128;
+            if (!z.records) {   // A in = in - P L^{-1} S in
+                IDC_TRY_CUDA(launch_axpby(1.0, z.in, 0.0, z.out, n, st));
+                IDC_TRY_CUDA(launch_axpby(-1.0, z.tmp, 1.0, z.out, n, st));
+            }
             if (z.restart_pending) {   // r = b - A x
                 IDC_TRY_CUDA(launch_axpby(1.0, z.b, -1.0, z.Vc(0), n, st));
-                IDC_TRY_CUDA(launch_dot(z.Vc(0), z.Vc(0), n, ds + 127, scratch, st));
+                IDC_TRY_CUDA(launch_dot(z.Vc(0), z.Vc(0), n, c.d_small + 127, c.d_small + 128, st));
             } else {                   // CGS2 against V_0 .. V_j, then |w|^2
                 const int j = z.j;
+                double *ds = c.d_small, *scratch = c.d_small + 128;
                 IDC_TRY_CUDA(launch_multidot(z.V, j + 1, n, z.Vc(j + 1), n, ds, scratch, st));
                 IDC_TRY_CUDA(launch_multiaxpy(z.Vc(j + 1), z.V, j + 1, n, ds, n, st));
                 IDC_TRY_CUDA(launch_multidot(z.V, j + 1, n, z.Vc(j + 1), n, ds + 64, scratch, st));
                 IDC_TRY_CUDA(launch_multiaxpy(z.Vc(j + 1), z.V, j + 1, n, ds + 64, n, st));
                 IDC_TRY_CUDA(launch_dot(z.Vc(j + 1), z.Vc(j + 1), n, ds + 127, scratch, st));
             }
+            double *ds = c.d_small;
             IDC_TRY_CUDA(cudaMemcpyAsync(c.h_small, ds, sizeof(double) * 128, cudaMemcpyDeviceToHost, st));
             IDC_TRY_CUDA(cudaMemcpyAsync(c.h_small + 128, d_err + p, sizeof(int), cudaMemcpyDeviceToHost, st));
         }
@@ -539,7 +595,10 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
         }
     }
     // psi = L^{-1}(S phi + Q) of every member in one batched sweep (in place: Q in, psi out)
-    for (auto &z : S) IDC_TRY_CUDA(launch_scatter_moments(z.c->dims(), z.c->d_sigma_s, z.x, z.scat, st));
+    for (size_t p = 0; p < M; ++p) {
+        IDC_TRY(scatter(S[p], S[p].x));
+        scats[p] = S[p].scat;
+    }
     IDC_TRY(sweep(srcs.data(), psi_inout, scats.data(), 1.0, nullptr, dt, precision));
     bool all = true;
     for (size_t p = 0; p < M; ++p) {

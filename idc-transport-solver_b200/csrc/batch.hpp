@@ -3,6 +3,7 @@
 
 #include "context.hpp"
 
+#include <array>
 #include <map>
 #include <utility>
 #include <vector>
@@ -15,9 +16,12 @@ public:
     Status add(Context *c);
     // per problem p (arrays indexed like `members`, entries nullable): outs[p] <- L^{-1}(srcs[p] +
     // scale phi_sc[p]), phis[p] <- P outs[p]; device pointers.  phi_sc[p] holds the scattering moments
-    // sigma_s phi / (4 pi) per cell (launch_scatter_moments), S phi without the ordinate broadcast
+    // sigma_s phi / (4 pi) per cell, S phi without the ordinate broadcast: launch_cell_records for members on the
+    // lane kernel (get_shape: warps 0), launch_scatter_moments for the modal one.  peierls (moments only): for members on
+    // the lane kernel phi_sc[p] is a moment vector x itself and phis[p] <- x - P L^{-1} S x
     Status sweep(const double *const *srcs, double *const *outs, const double *const *phi_sc, double scale,
-                 double *const *phis, double dt, int precision, const std::vector<char> *active = nullptr);
+                 double *const *phis, double dt, int precision, const std::vector<char> *active = nullptr,
+                 bool peierls = false);
     // GMRES(restart) on every member's Peierls system at once (the algorithm of Context::gmres_peierls, with
     // each member's preconditioner): every Krylov step sweeps all unconverged members in one batched sweep,
     // their Arnoldi steps and DSA applications run on the device per member, with one host synchronisation
@@ -36,7 +40,7 @@ public:
 
 private:
     struct Group {
-        int P = 0, seg = 0, wn = 0, G = 0, precision = -1, n_items = 0, grid = 0;
+        int P = 0, seg = 0, wn = 0, lane_wn = 0, G = 0, precision = -1, n_items = 0, grid = 0;
         size_t smem = 0;
         std::vector<int> members, items_per_rb;
         SweepItem *d_items = nullptr;
@@ -47,10 +51,11 @@ private:
         cudaEvent_t upload_done = nullptr;       // the last upload has read h_table
         std::vector<double *> trace, phi_part, inflow;
         std::vector<size_t> trace_len;
+        std::vector<std::array<int, 5>> slot_begin;   // per member: the quadrants' partial-moment slots
     };
     Status build_group(Group &g, int precision);
     Status launch_group(Group &g, const double *const *srcs, double *const *outs, const double *const *phi_sc,
-                        double scale, double *const *phis, double dt, const std::vector<char> *active);
+                        double scale, double *const *phis, double dt, const std::vector<char> *active, bool peierls);
     void release();
     // every group launches on the first member's stream, so that one synchronisation and one event pair
     // cover the whole batched sweep

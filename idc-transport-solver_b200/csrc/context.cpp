@@ -56,8 +56,10 @@ Context::~Context() {
     cudaFree(d_w);
     cudaFree(d_sigma_t);
     cudaFree(d_sigma_s);
-    cudaFree(other_sched_.d_items);
-    cudaFree(other_sched_.d_trace);
+    for (auto &o : sched_slots_) {
+        cudaFree(o.d_items);
+        cudaFree(o.d_trace);
+    }
     cudaFree(d_sig_mom_);
     cudaFree(d_tens_t_);
     cudaFree(d_tens_s_);
@@ -615,27 +617,30 @@ static void choose_warp_tiling(int qmax, int user_G, int user_rows, int max_wn, 
     *wn_out = wn;
 }
 
-// Work items in row-block-major order: (row block, quadrant, ordinate chunk).
 void Context::use_schedule(int variant) {
     if (variant == sched_variant_) return;
-    ScheduleSlot &o = other_sched_;
-    std::swap(tiling, o.tiling);
-    std::swap(d_items, o.d_items);
-    std::swap(d_trace, o.d_trace);
-    std::swap(trace_len, o.trace_len);
-    std::swap(smem, o.smem);
-    std::swap(n_items, o.n_items);
-    std::swap(items_per_rb, o.items_per_rb);
-    for (int k = 0; k < 5; ++k) std::swap(quad_slots[k], o.quad_slots[k]);
-    std::swap(seg, o.seg);
-    std::swap(wn, o.wn);
-    std::swap(active, o.active);
-    std::swap(grid, o.grid);
-    std::swap(block, o.block);
-    std::swap(occupancy_precision, o.occupancy_precision);
+    auto swap_with = [&](ScheduleSlot &o) {
+        std::swap(tiling, o.tiling);
+        std::swap(d_items, o.d_items);
+        std::swap(d_trace, o.d_trace);
+        std::swap(trace_len, o.trace_len);
+        std::swap(smem, o.smem);
+        std::swap(n_items, o.n_items);
+        std::swap(items_per_rb, o.items_per_rb);
+        for (int k = 0; k < 5; ++k) std::swap(quad_slots[k], o.quad_slots[k]);
+        std::swap(seg, o.seg);
+        std::swap(wn, o.wn);
+        std::swap(active, o.active);
+        std::swap(grid, o.grid);
+        std::swap(block, o.block);
+        std::swap(occupancy_precision, o.occupancy_precision);
+    };
+    swap_with(sched_slots_[sched_variant_]);
+    swap_with(sched_slots_[variant]);
     sched_variant_ = variant;
 }
 
+// Work items in row-block-major order: (row block, quadrant, ordinate chunk).
 Status Context::build_schedule(int precision) {
     if (n_items > 0 && occupancy_precision == precision) return Status::ok();
     // the lane kernel's schedule does not depend on the precision (the same tiling rules, traces and grid for
@@ -653,7 +658,7 @@ Status Context::build_schedule(int precision) {
     const int max_wn = active == kModal ? sweep_modal_max_wn(P) : active == kLane ? 1 : 7;
     const bool modal_like = active == kModal || active == kLane;
     // a fixed or autotuned tile shape is the full sweeps'; the moments-only sweeps keep the default rule
-    if (use_warp_kernel && tune_seg > 0 && sched_variant_ == 0) {
+    if (use_warp_kernel && tune_seg > 0 && sched_variant_ != 1) {
         seg = tune_seg;
         if (active == kLane && !sweep_lane_supports(P, precision, seg)) seg = 16;
         wn = tune_wn > 0 ? std::min(tune_wn, max_wn) : (active == kModal ? sweep_modal_default_wn(P) : 1);
@@ -664,11 +669,11 @@ Status Context::build_schedule(int precision) {
     } else if (use_warp_kernel) {
         choose_warp_tiling(qmax, user_G, user_R, max_wn, active == kModal ? sweep_modal_default_wn(P) : max_wn,
                            modal_like, &G, &seg, &wn);
-        if (active == kLane && sched_variant_ == 0 && user_G == 0 && user_R == 0 && (P == 3 || (P == 2 && qmax <= 24))) {
-            // full lane sweeps: at DG degree 2 16-wide segments (fewer row blocks, 16-wide moment sums) were the
-            // fastest at S8, S12 and S16 on 256^2 grids; at degree 1 8-wide ones for up to 24 ordinates per quadrant
-            // (S8, S12: 4-7% ahead of 4-wide, also on the 64^2 lattice), while S16's 36 keep the 4-wide rule
-            seg = P == 3 ? 16 : 8;
+        if (active == kLane && sched_variant_ != 1 && user_G == 0 && user_R == 0 && P == 3) {
+            // full sweeps at DG degree 2: 16-wide segments (fewer partial moments, and their sums from shared memory
+            // instead of shuffles); B200, 256x256 S16: 671 us, 722 with 8, 697 with 4; 192x160 S12 359, 379 with 4.  At
+            // degrees 0 and 1, and for the moments-only sweeps, the narrowest: 512x512 Q1 S12 753, 776 with 8
+            seg = 16;
             const int nch = (qmax + seg - 1) / seg;
             G = (qmax + nch - 1) / nch;
         }
@@ -691,6 +696,15 @@ Status Context::build_schedule(int precision) {
         R = user_R > 0 ? user_R : std::max(1, std::min(16, max_threads / G));
         if (G * R > max_threads) R = std::max(1, max_threads / G);
         if (R > ny) R = (int)ny;
+    }
+    if (active == kLane) {
+        int64_t chains = 0;
+        for (int k = 0; k < 4; ++k) chains += ((quad[k + 1] - quad[k]) + G - 1) / G;
+        wn = sweep_lane_warps(P, seg, sched_variant_ == 2, num_sms, [&](int w) {
+            const int64_t rows = w * (32 / seg);
+            return chains * ((ny + rows - 1) / rows);
+        });
+        R = wn * (32 / seg);
     }
     tiling.G = G;
     tiling.R = R;
@@ -762,9 +776,9 @@ Status Context::build_schedule(int precision) {
 
     int per_sm = 0;
     if (active == kLane) {
-        block = sweep_lane_warps() * 32;
-        smem = 0;   // fixed per kernel instance (set by the launcher)
-        IDC_TRY_CUDA(sweep_lane_occupancy(P, seg, false, &per_sm));
+        block = (wn + 1) * 32;
+        smem = 0;   // set by the launcher
+        IDC_TRY_CUDA(sweep_lane_occupancy(P, seg, wn, sched_variant_ == 2, &per_sm));
     } else if (active == kModal) {
         block = sweep_modal_threads(P, wn);
         smem = sweep_modal_smem_bytes(P, precision, wn, G, seg);
@@ -779,10 +793,7 @@ Status Context::build_schedule(int precision) {
         IDC_TRY_CUDA(sweep_occupancy(P, precision, block, smem, &per_sm));
     }
     if (per_sm < 1) return bad(IDC_ERR_UNSUPPORTED, "sweep kernel does not fit on an SM with this tiling");
-    if (active == kLane)   // one item per warp at a time
-        grid = std::min((n_items + sweep_lane_warps() - 1) / sweep_lane_warps(), per_sm * num_sms);
-    else
-        grid = std::min(n_items, per_sm * num_sms);
+    grid = std::min(n_items, per_sm * num_sms);
     occupancy_precision = precision;
     return Status::ok();
 }
@@ -843,9 +854,10 @@ Status Context::check_device_error() {
         IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 1, 0, sizeof(int), stream));
         if (d_trace)
             IDC_TRY_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long *>(d_trace), trace_len, kTraceSentinel, stream));
-        if (other_sched_.d_trace)   // the other variant's schedule: its sweeps may have been the abandoned ones
-            IDC_TRY_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long *>(other_sched_.d_trace),
-                                         other_sched_.trace_len, kTraceSentinel, stream));
+        for (auto &o : sched_slots_)   // the other variants' schedules: their sweeps may have been the abandoned ones
+            if (o.d_trace)
+                IDC_TRY_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long *>(o.d_trace), o.trace_len,
+                                             kTraceSentinel, stream));
         IDC_TRY_CUDA(cudaStreamSynchronize(stream));
         return bad(IDC_ERR_TIMEOUT, "a device-side wait gave up (bounded spin); the sweep was abandoned");
     }
@@ -854,7 +866,7 @@ Status Context::check_device_error() {
 
 Status Context::sweep(const double *src, double *out, double dt, double *phi, int precision,
                       const double *phi_scatter, double scatter_scale, bool adjoint, const double *src2,
-                      double src2_scale) {
+                      double src2_scale, const double *minuend) {
     if (!have_ordinates) return bad(IDC_ERR_STATE, "sweep before idc_set_ordinates");
     if (!have_sigma) return bad(IDC_ERR_STATE, "sweep before idc_set_sigma");
     if (precision < 0 || precision > 2) return bad(IDC_ERR_ARG, "unknown precision");
@@ -876,7 +888,10 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
     }
     if (reflect_mask && !in_reflect_)
         return sweep_reflecting(src, out, dt, phi, precision, phi_scatter, scatter_scale, adjoint, src2);
-    use_schedule((!src && !out && phi && !adjoint && !src2 && moments_fast_path) ? 1 : 0);
+    const bool lane = kernel_for(precision) == kLane;
+    use_schedule(!src && !out && phi && !src2 && moments_fast_path && (lane || !adjoint) ? 1
+                 : src2 && lane && precision == IDC_PREC_FP64 && P == 3                  ? 2
+                                                                                         : 0);
     IDC_TRY(build_schedule(precision));
     IDC_TRY_CUDA(cudaSetDevice(device));
 
@@ -960,12 +975,13 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
         a.phi_slot_stride = phi_len();
     }
 
-    // moments-only forward sweeps (the Krylov iterations) on the lane kernel: no per-ordinate transforms
-    const bool phi_only = active == kLane && !src && !out && phi && !adjoint && !src2 && a.phi_part && moments_fast_path;
+    // moments-only sweeps (the Krylov iterations) on the lane kernel: no per-ordinate transforms
+    const bool phi_only = active == kLane && !src && !out && phi && !src2 && a.phi_part && moments_fast_path;
 
     // queue head and progress flags start at zero; the error word is kept until checked
     IDC_TRY_CUDA(cudaMemsetAsync(d_sync, 0, sizeof(int), stream));
-    IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 2, 0, sizeof(int) * n_items, stream));
+    if (active == kRowSync)   // the only kernel with progress flags
+        IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 2, 0, sizeof(int) * n_items, stream));
     if (a.phi) IDC_TRY_CUDA(cudaMemsetAsync(phi, 0, sizeof(double) * phi_len(), stream));
     if (active != kModal && active != kLane && !capturing) IDC_TRY_CUDA(cudaEventRecord(ev0, stream));
     if (active == kModal || active == kLane) {
@@ -983,22 +999,8 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
             launches += 1;
             a.inflow = d_inflow;
         }
-        if (phi_scatter && !adjoint) {   // the scattering source's moments, once per cell instead of per ordinate
-            if (scat_len < phi_len()) {
-                if (capturing) return bad(IDC_ERR_STATE, "scattering buffer allocation inside a stream capture");
-                cudaFree(d_scat);
-                d_scat = nullptr;
-                scat_len = 0;
-                IDC_TRY_CUDA(cudaMalloc(&d_scat, sizeof(double) * phi_len()));
-                scat_len = phi_len();
-            }
-            IDC_TRY_CUDA(launch_scatter_moments(dims(), d_sigma_s, phi_scatter, d_scat, stream));
-            launches += 1;
-            a.phi_scatter = d_scat;
-            a.sigma_s = nullptr;
-        }
         if (phi_only) {   // the scattering source in the packed modal basis, once per (cell, quadrant)
-            const size_t need = sig_len() * 4 * N;
+            const size_t need = sig_len() * 4 * cell_record_doubles(P);
             if (msrc_len < need) {
                 if (capturing) return bad(IDC_ERR_STATE, "modal source buffer allocation inside a stream capture");
                 cudaFree(d_msrc);
@@ -1007,10 +1009,34 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
                 IDC_TRY_CUDA(cudaMalloc(&d_msrc, sizeof(double) * need));
                 msrc_len = need;
             }
-            IDC_TRY_CUDA(launch_modal_sources(dims(), a.phi_scatter, scatter_scale, d_msrc, stream));
+            IDC_TRY_CUDA(launch_modal_sources(dims(), d_sigma_t, adjoint ? nullptr : d_sigma_s, phi_scatter,
+                                              adjoint ? 1.0 : scatter_scale, adjoint, d_msrc, stream));
             launches += 1;
             a.modal_src = d_msrc;
             a.phi_scatter = nullptr;
+        } else if (phi_scatter && (active == kLane || !adjoint)) {
+            // the scattering source's moments, once per cell instead of per ordinate (the lane kernel's in records
+            // with sigma_t; its transposed sweep's hold mu)
+            const size_t need = sig_len() * cell_record_doubles(P);
+            if (scat_len < need) {
+                if (capturing) return bad(IDC_ERR_STATE, "scattering buffer allocation inside a stream capture");
+                cudaFree(d_scat);
+                d_scat = nullptr;
+                scat_len = 0;
+                IDC_TRY_CUDA(cudaMalloc(&d_scat, sizeof(double) * need));
+                scat_len = need;
+            }
+            if (active == kLane) {
+                IDC_TRY_CUDA(launch_cell_records(dims(), d_sigma_t, adjoint ? nullptr : d_sigma_s, phi_scatter, d_scat,
+                                                 stream));
+                a.cell_rec = d_scat;
+                a.phi_scatter = nullptr;
+            } else {
+                IDC_TRY_CUDA(launch_scatter_moments(dims(), d_sigma_s, phi_scatter, d_scat, stream));
+                a.phi_scatter = d_scat;
+            }
+            launches += 1;
+            a.sigma_s = nullptr;
         }
         if (!capturing) IDC_TRY_CUDA(cudaEventRecord(ev0, stream));   // the timing covers the sweep kernel alone
         if (active == kLane)
@@ -1024,7 +1050,7 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
     if (!capturing) IDC_TRY_CUDA(cudaEventRecord(ev1, stream));
     launches += 1;
     if (a.phi_part && phi_only) {
-        IDC_TRY_CUDA(launch_reduce_modal_partials(dims(), d_phi_part, quad_slots, phi_len(), phi, stream));
+        IDC_TRY_CUDA(launch_reduce_modal_partials(dims(), d_phi_part, quad_slots, phi_len(), adjoint, minuend, phi, stream));
         launches += 1;
     } else if (a.phi_part && !skip_reduce_) {
         IDC_TRY_CUDA(launch_reduce_phi_partials(dims(), d_phi_part, items_per_rb, phi_len(), phi, stream));

@@ -41,9 +41,10 @@ public:
     // Sweep: out <- L^{-1} (src [+ scale * S phi_scatter]); phi (nullable) <- P out.  src may equal out.
     // src2 (modal kernel, forward): the source is src + src2_scale * src2 on interior cells, combined by the
     // sweep's aux warps (or, when its stages do not fit in shared memory, by a kernel into a scratch array)
+    // minuend (moments-only sweeps on the lane kernel, no all-reduce hook): phi <- minuend - P out instead
     Status sweep(const double *src, double *out, double dt, double *phi, int precision,
                  const double *phi_scatter = nullptr, double scatter_scale = 1.0, bool adjoint = false,
-                 const double *src2 = nullptr, double src2_scale = 0.0);
+                 const double *src2 = nullptr, double src2_scale = 0.0, const double *minuend = nullptr);
     // count out-of-place sweeps of HOST arrays (srcs[k] -> outs[k] interior cells, phis[k] if phis), the
     // upload of step k+1, the sweep of step k and the download of step k-1 overlapped on three streams
     // with double-buffered device arrays
@@ -126,8 +127,6 @@ public:
     double dx = 0, dy = 0;
     int device = 0;
     int num_sms = 0;
-    int lane_src2_blocks_[2] = {-1, -1};   // resident blocks per SM of the lane kernel's second-source
-                                           // instance at DG degree 1, segments 8 and 4 (-1: not queried yet)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -168,10 +167,10 @@ public:
     double *d_trace = nullptr;     // warp / modal kernel: per-item last-row traces (sentinel-armed)
     double *d_inflow = nullptr;    // modal kernel: inflow traces of the ghost cells
     size_t inflow_len = 0;
-    double *d_scat = nullptr;      // modal kernel: the fused scattering source's moments sigma_s phi / (4 pi)
+    double *d_scat = nullptr;      // lane kernel: cell records; modal kernel: the moments sigma_s phi / (4 pi)
     size_t scat_len = 0;
     double *d_src2mix = nullptr;   // src + scale src2 when the second source's stages do not fit
-    double *d_msrc = nullptr;      // lane kernel, moments-only sweeps: packed modal sources [(nx+2)(ny+2)][4][N]
+    double *d_msrc = nullptr;      // lane kernel, moments-only sweeps: packed modal sources [(nx+2)(ny+2)][4][record]
     size_t msrc_len = 0;
     bool moments_fast_path = true;
     int quad_slots[5] = {0, 0, 0, 0, 0};   // partial-moment slots of each quadrant within a row block
@@ -184,10 +183,11 @@ public:
     size_t smem = 0;
     int occupancy_precision = -1;
     size_t sync_cap_ = 0;          // ints allocated at d_sync (shared by both schedules below)
-    // Two cached schedules, one per sweep variant: 0 = sweeps with a source or a psi output, 1 = the moments-only
-    // Krylov sweeps (no source, psi not stored).  They want different tile widths (the full lane sweep at DG
+    // Cached schedules, one per sweep variant: 0 = sweeps with a source or a psi output, 1 = the moments-only Krylov
+    // sweeps (no source, psi not stored), 2 = sweeps with a second source at DG degree 2 on the lane kernel (whose
+    // stages leave room for fewer warps per block).  They want different tile widths (the full lane sweep at DG
     // degree 2 is fastest with 16-wide segments, the moments-only one with narrow ones), and GMRES alternates
-    // between them, so the members above hold the current variant's schedule and `other_sched_` the other's;
+    // between them, so the members above hold the current variant's schedule and `sched_slots_` the others';
     // `use_schedule` swaps them.  d_sync (the error word and progress flags) is shared.
     struct ScheduleSlot {
         SweepTiling tiling{};
@@ -197,14 +197,16 @@ public:
         int n_items = 0, items_per_rb = 0, quad_slots[5] = {0, 0, 0, 0, 0}, seg = 0, wn = 0, active = 3, grid = 0,
             block = 0, occupancy_precision = -1;
     };
-    ScheduleSlot other_sched_;
+    ScheduleSlot sched_slots_[3];   // the variants not current (the current one's slot is empty)
     int sched_variant_ = 0;
     void use_schedule(int variant);
     void invalidate_schedules() {
         n_items = 0;
         occupancy_precision = -1;
-        other_sched_.n_items = 0;
-        other_sched_.occupancy_precision = -1;
+        for (auto &o : sched_slots_) {
+            o.n_items = 0;
+            o.occupancy_precision = -1;
+        }
     }
 
     float last_sweep_ms = 0.f;

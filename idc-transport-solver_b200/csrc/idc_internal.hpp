@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cstddef>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -76,10 +77,18 @@ struct SweepArgs {
                                // at once; nothing of it is read or written)
     int quad_mask;             // lane kernel: quadrants swept by this launch (bit k = quadrant k), 0 = all; items of
                                // the others return at once (reflecting boundaries sweep the quadrants in sequence)
-    const double *modal_src;   // lane kernel, moments-only forward sweeps: the packed modal source of every
-                               // (cell, quadrant), [(nx+2)(ny+2)][4][N] (launch_modal_sources), or null; the
-                               // partial moments are then packed modal sums (launch_reduce_modal_partials)
+    const double *modal_src;   // lane kernel, moments-only sweeps: the packed modal source and sigma_t of every
+                               // (cell, quadrant), [(nx+2)(ny+2)][4][cell_record_doubles] (launch_modal_sources),
+                               // or null; the partial moments are then packed modal sums
+                               // (launch_reduce_modal_partials)
+    const double *cell_rec;    // lane kernel, the other sweeps with a scattering term: the scattering moments (mu for
+                               // the transposed sweep) and sigma_t of every cell, [(nx+2)(ny+2)][cell_record_doubles]
+                               // (launch_cell_records), or null
+    int slot_begin[6];         // batched moments-only launch: the partial-moment slots of each quadrant (5 bounds)
 };
+
+// Doubles of a cell's record: N moments, sigma_t, rounded up to whole 16-byte words.
+__host__ __device__ constexpr int cell_record_doubles(int P) { return (P * P + 2) / 2 * 2; }
 
 // Launch geometry picked by the host (autotuner or defaults).
 struct SweepTiling {
@@ -100,19 +109,21 @@ size_t sweep_warp_smem_bytes(int P, int wn, int G, int seg);
 constexpr int kWarpRingSlots = 8;
 constexpr int kModalSolutionSlots = 4;   // modal kernel: step results in flight per compute warp
 
-// Lane-pipelined sweep kernel (sweep_lane.cu): every warp an independent worker on one item of 32/seg rows
-// (R = 32/seg, G <= seg); FP64 forward (optionally with src2), transposed or moments-only, and FP32
-// (IDC_PREC_FP32) forward or moments-only sweeps; `grid` thread blocks of
-// sweep_lane_warps() warps.  Same arguments and trace protocol as the modal kernel.
+// Lane-pipelined sweep kernel (sweep_lane.cu): an item is wn * 32/seg rows (R; G <= seg), one row block per warp of
+// a thread block of wn + 1 warps; FP64 forward (optionally with src2), transposed or moments-only, and FP32
+// (IDC_PREC_FP32) forward or moments-only sweeps.  Same arguments and trace protocol as the modal kernel.
 bool sweep_lane_supports(int P, int precision, int seg);
-int sweep_lane_warps();
+// warps per block (wn) for a launch of row_blocks(w) items with w warps per block
+int sweep_lane_warps(int P, int seg, bool src2, int num_sms, const std::function<int64_t(int)> &row_blocks);
 // A batch's FP64 forward sweep on the lane kernel: the items of several problems of one DG degree (`table`:
 // one SweepArgs per problem on the device; items name their problem and carry problem-local indices)
-cudaError_t launch_sweep_lane_batched(int P, const SweepArgs &args, const SweepArgs *table, int grid,
-                                      cudaStream_t stream);
-cudaError_t sweep_lane_batched_occupancy(int P, int seg, int *blocks_per_sm);
+// moments_only: one Peierls operator application per problem, phi = phi_scatter - P L^{-1} S phi_scatter, in three
+// launches for all `members` (each problem's modal_src is written first)
+cudaError_t launch_sweep_lane_batched(int P, const SweepArgs &args, const SweepArgs *table, int members, bool moments_only,
+                                      int grid, cudaStream_t stream);
+cudaError_t sweep_lane_batched_occupancy(int P, int seg, int warps, int *blocks_per_sm);
 cudaError_t launch_sweep_lane(int P, int precision, const SweepArgs &args, int grid, cudaStream_t stream);
-cudaError_t sweep_lane_occupancy(int P, int seg, bool src2, int *blocks_per_sm);
+cudaError_t sweep_lane_occupancy(int P, int seg, int warps, bool src2, int *blocks_per_sm);
 
 // Modal sweep kernel (sweep_modal.cu): same arguments as the warp kernel plus `inflow`, traces of P values.
 cudaError_t launch_sweep_modal(int P, int precision, const SweepArgs &args, int grid, size_t smem, cudaStream_t stream);
@@ -154,16 +165,21 @@ struct GridDims {
     int nx, ny, nq, P;
     double dx, dy;
 };
-// Moments-only forward sweeps (no source array, psi not stored) on the lane kernel: the source of a cell is
-// the isotropic scattering source, the same for every ordinate of a quadrant, so its packed modal transform
-// is formed once per (cell, quadrant): out[(cell * 4 + k) * N + m] = W flip_k(scale * moments) W^T (moments
-// = sigma_s phi / (4 pi) of launch_scatter_moments, null for none).  The sweep then sums w_q Z in the packed
-// basis per ordinate chunk, and the reduction transforms each quadrant's sum back once per cell:
-// phi = sum_k flip_k(V (sum_{slots of k} part) V^T), slots [slot_begin[k], slot_begin[k+1]) of quadrant k,
-// interior cells in a fixed order, ghost cells zero.
-cudaError_t launch_modal_sources(const GridDims &g, const double *moments, double scale, double *out, cudaStream_t s);
+// Moments-only sweeps (no source array, psi not stored) on the lane kernel: the source of a cell is the isotropic
+// scattering source, the same for every ordinate of a quadrant (times w_q for the transposed sweep), so its packed
+// modal transform is formed once per (cell, quadrant): out[(cell * 4 + k) * cell_record_doubles + m] =
+// W flip_k(scale * sigma_s phi / (4 pi)) W^T (phi itself with sigma_s null; zero with phi null), then sigma_t.  The
+// sweep sums w_q Z (Z for the transposed sweep) in the packed basis per ordinate chunk, and the reduction transforms
+// each quadrant's sum back once per cell: phi = sum_k flip_k(V (sum_{slots of k} part) V^T), slots
+// [slot_begin[k], slot_begin[k+1]) of quadrant k, interior cells in a fixed order, ghost cells zero; with
+// `minuend` x the output is x - phi (the Peierls operator's).
+cudaError_t launch_modal_sources(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
+                                 double scale, bool adjoint, double *out, cudaStream_t s);
 cudaError_t launch_reduce_modal_partials(const GridDims &g, const double *part, const int slot_begin[5], size_t stride,
-                                         double *phi, cudaStream_t s);
+                                         bool adjoint, const double *minuend, double *phi, cudaStream_t s);
+// The records of SweepArgs::cell_rec: sigma_s phi / (4 pi) (phi itself with sigma_s null), then sigma_t.
+cudaError_t launch_cell_records(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
+                                double *out, cudaStream_t s);
 cudaError_t launch_pmv(const GridDims &g, double alpha, double beta, const double *w, const double *psi,
                        double *phi, cudaStream_t s);
 cudaError_t launch_smv(const GridDims &g, double alpha, double beta, const double *sigma_s, const double *phi,

@@ -44,6 +44,8 @@ Status Context::dot_host(const double *x, const double *y, size_t n, double *out
 // y = x - P L^{-1} S x  (IPLS, PETScPeierlsSolver.cpp:529-572): one sweep with no angular source and
 // vacuum inflow, the scattering source built from x on the fly, psi not stored.
 Status Context::apply_peierls(const double *x, double *y, double *tmp_phi, double dt, int precision) {
+    if (kernel_for(precision) == kLane && moments_fast_path && !allreduce_fn && !reflect_mask)   // x - in the reduction
+        return sweep(nullptr, nullptr, dt, y, precision, x, 1.0, false, nullptr, 0.0, x);
     IDC_TRY(sweep(nullptr, nullptr, dt, tmp_phi, precision, x, 1.0));
     IDC_TRY_CUDA(launch_axpby(1.0, x, 0.0, y, phi_len(), stream));
     IDC_TRY_CUDA(launch_axpby(-1.0, tmp_phi, 1.0, y, phi_len(), stream));

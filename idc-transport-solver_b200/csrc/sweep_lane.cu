@@ -2,6 +2,8 @@
 // and the occupancy query.  The kernel is in sweep_lane_impl.cuh.
 #include "sweep_lane_impl.cuh"
 
+#include <cmath>
+
 namespace idc {
 
 namespace {
@@ -26,37 +28,84 @@ cudaError_t launch_dir(const SweepArgs &args, int grid, cudaStream_t stream, boo
         }
         return launch_p<P, false, false, false, float>(args, grid, stream);
     }
-    if (args.modal_src) {   // moments-only forward sweep
-        if (args.adjoint || args.src2 || args.src || args.out || !args.phi_part) return cudaErrorInvalidValue;
-        return launch_p<P, false, false, true>(args, grid, stream);
+    if (args.modal_src) {   // moments-only sweep
+        if (args.src2 || args.src || args.out || !args.phi_part) return cudaErrorInvalidValue;
+        return args.adjoint ? launch_p<P, true, false, true>(args, grid, stream)
+                            : launch_p<P, false, false, true>(args, grid, stream);
     }
     if (args.adjoint) return args.src2 ? cudaErrorInvalidValue : launch_p<P, true, false>(args, grid, stream);
     return args.src2 ? launch_p<P, false, true>(args, grid, stream) : launch_p<P, false, false>(args, grid, stream);
 }
 
-// Packed modal source of every interior (cell, quadrant) for the moments-only sweep (see idc_internal.hpp).
-template <int P>
-__global__ void modal_sources_kernel(GridDims g, const double *__restrict__ mom, double scale, double *__restrict__ out) {
-    constexpr int N = P * P;
-    const size_t total = (size_t)g.nx * g.ny * 4;
+// Packed modal source (of the forward or the transposed operator) and sigma_t of every interior (cell, quadrant) for
+// the moments-only sweep (see idc_internal.hpp): sigma_s phi / (4 pi) scaled (rounded as scatter_moments_kernel rounds
+// it), or phi itself without sigma_s.
+template <int P, bool ADJ>
+__device__ __forceinline__ void modal_sources(int nx, int ny, const double *__restrict__ sigma_t,
+                                              const double *__restrict__ sigma_s, const double *__restrict__ phi,
+                                              double scale, double *__restrict__ out) {
+    constexpr int N = P * P, RD = cell_record_doubles(P);
+    const size_t total = (size_t)nx * ny * 4;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const int k = (int)(t % 4);
         const size_t cell = t / 4;
-        const int i = 1 + (int)(cell / g.ny), j = 1 + (int)(cell % g.ny);
-        const size_t cidx = (size_t)i * (g.ny + 2) + j;
+        const int i = 1 + (int)(cell / ny), j = 1 + (int)(cell % ny);
+        const size_t cidx = (size_t)i * (ny + 2) + j;
+        const double ss = sigma_s ? sigma_s[cidx] : 0.0;
         double v[N], S[N];
 #pragma unroll
-        for (int m = 0; m < N; ++m) v[m] = mom ? scale * mom[cidx * N + m] : 0.0;
+        for (int m = 0; m < N; ++m) {
+            v[m] = phi ? phi[cidx * N + m] : 0.0;
+            if (sigma_s) v[m] = (ss * v[m]) / (4.0 * M_PI);
+            v[m] *= scale;
+        }
         const bool xn = k >= 2, yn = (k & 1) != 0;
 #pragma unroll
         for (int m = 0; m < N; ++m) {   // the quadrant's sign flip x(d,e) -> sx^d sy^e x(d,e)
             const int d = m / P, e = m % P;
             if (((d & 1) && xn) != ((e & 1) && yn)) v[m] = -v[m];
         }
-        modal_forward<P, false, false, double, false>(S, v);
-        double *o = out + (cidx * 4 + k) * N;
+        modal_forward<P, false, false, double, ADJ>(S, v);
+        double *o = out + (cidx * 4 + k) * RD;
 #pragma unroll
         for (int m = 0; m < N; ++m) o[m] = S[m];
+        o[N] = sigma_t[cidx];
+    }
+}
+
+template <int P, bool ADJ>
+__global__ void modal_sources_kernel(GridDims g, const double *__restrict__ sigma_t, const double *__restrict__ sigma_s,
+                                     const double *__restrict__ phi, double scale, double *__restrict__ out) {
+    modal_sources<P, ADJ>(g.nx, g.ny, sigma_t, sigma_s, phi, scale, out);
+}
+// every problem of a batch's table (grid.y) that is not left out
+template <int P>
+__global__ void modal_sources_batched_kernel(const SweepArgs *__restrict__ table) {
+    const SweepArgs &a = table[blockIdx.y];
+    if (!a.skip)
+        modal_sources<P, false>(a.nx, a.ny, a.sigma_t, a.sigma_s, a.phi_scatter, a.scatter_scale,
+                                const_cast<double *>(a.modal_src));
+}
+
+// The records of every interior cell: sigma_s phi / (4 pi) (or phi itself without sigma_s), sigma_t.
+template <int P>
+__global__ void cell_records_kernel(GridDims g, const double *__restrict__ sigma_t, const double *__restrict__ sigma_s,
+                                    const double *__restrict__ phi, double *__restrict__ out) {
+    constexpr int N = P * P, RD = cell_record_doubles(P);
+    const size_t total = (size_t)g.nx * g.ny * RD;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+        const int m = (int)(t % RD);
+        const size_t cell = t / RD;
+        const int i = 1 + (int)(cell / g.ny), j = 1 + (int)(cell % g.ny);
+        const size_t cidx = (size_t)i * (g.ny + 2) + j;
+        double v = 0.0;
+        if (m < N) {
+            v = phi[cidx * N + m];
+            if (sigma_s) v = (sigma_s[cidx] * v) / (4.0 * M_PI);
+        } else if (m == N) {
+            v = sigma_t[cidx];
+        }
+        out[cidx * RD + m] = v;
     }
 }
 
@@ -65,18 +114,19 @@ __global__ void modal_sources_kernel(GridDims g, const double *__restrict__ mom,
 struct SlotBounds {
     int b[5];
 };
-template <int P>
-__global__ void reduce_modal_partials_kernel(GridDims g, const double *__restrict__ part, SlotBounds sb, size_t stride,
-                                             double *__restrict__ phi) {
+template <int P, bool ADJ>
+__device__ __forceinline__ void reduce_modal_partials(int nx, int ny, const double *__restrict__ part, const SlotBounds &sb,
+                                                      size_t stride, const double *__restrict__ minuend,
+                                                      double *__restrict__ phi) {
     constexpr int N = P * P;
-    const size_t total = (size_t)(g.nx + 2) * (g.ny + 2);
+    const size_t total = (size_t)(nx + 2) * (ny + 2);
     for (size_t cidx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; cidx < total;
          cidx += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(cidx / (g.ny + 2)), j = (int)(cidx % (g.ny + 2));
+        const int i = (int)(cidx / (ny + 2)), j = (int)(cidx % (ny + 2));
         double acc[N];
 #pragma unroll
         for (int m = 0; m < N; ++m) acc[m] = 0.0;
-        if (i >= 1 && i <= g.nx && j >= 1 && j <= g.ny) {
+        if (i >= 1 && i <= nx && j >= 1 && j <= ny) {
             for (int k = 0; k < 4; ++k) {
                 if (sb.b[k + 1] == sb.b[k]) continue;
                 double M[N], x[N];
@@ -85,7 +135,7 @@ __global__ void reduce_modal_partials_kernel(GridDims g, const double *__restric
                 for (int sl = sb.b[k]; sl < sb.b[k + 1]; ++sl)
 #pragma unroll
                     for (int m = 0; m < N; ++m) M[m] += part[(size_t)sl * stride + cidx * N + m];
-                modal_backward<P, false, false, double, false>(x, M);
+                modal_backward<P, false, false, double, ADJ>(x, M);
                 const bool xn = k >= 2, yn = (k & 1) != 0;
 #pragma unroll
                 for (int m = 0; m < N; ++m) {
@@ -95,8 +145,21 @@ __global__ void reduce_modal_partials_kernel(GridDims g, const double *__restric
             }
         }
 #pragma unroll
-        for (int m = 0; m < N; ++m) phi[cidx * N + m] = acc[m];
+        for (int m = 0; m < N; ++m) phi[cidx * N + m] = minuend ? minuend[cidx * N + m] - acc[m] : acc[m];
     }
+}
+template <int P, bool ADJ>
+__global__ void reduce_modal_partials_kernel(GridDims g, const double *__restrict__ part, SlotBounds sb, size_t stride,
+                                             const double *__restrict__ minuend, double *__restrict__ phi) {
+    reduce_modal_partials<P, ADJ>(g.nx, g.ny, part, sb, stride, minuend, phi);
+}
+template <int P>
+__global__ void reduce_modal_batched_kernel(const SweepArgs *__restrict__ table) {
+    const SweepArgs &a = table[blockIdx.y];
+    if (a.skip) return;
+    SlotBounds sb;
+    for (int k = 0; k < 5; ++k) sb.b[k] = a.slot_begin[k];
+    reduce_modal_partials<P, false>(a.nx, a.ny, a.phi_part, sb, a.phi_slot_stride, a.phi_scatter, a.phi);
 }
 
 int blocks_for(size_t n) {
@@ -105,13 +168,18 @@ int blocks_for(size_t n) {
 }
 
 template <int P>
-cudaError_t occ_p(int seg, bool src2, int *n) {
+cudaError_t occ_p(int seg, int warps, bool src2, int *n) {
     switch (seg) {
-        case 4: return src2 ? lane::occupancy<P, 4, false, true>(n) : lane::occupancy<P, 4, false, false>(n);
-        case 8: return src2 ? lane::occupancy<P, 8, false, true>(n) : lane::occupancy<P, 8, false, false>(n);
-        case 16: return src2 ? lane::occupancy<P, 16, false, true>(n) : lane::occupancy<P, 16, false, false>(n);
+        case 4: return src2 ? lane::occupancy<P, 4, false, true>(warps, n) : lane::occupancy<P, 4, false, false>(warps, n);
+        case 8: return src2 ? lane::occupancy<P, 8, false, true>(warps, n) : lane::occupancy<P, 8, false, false>(warps, n);
+        case 16: return src2 ? lane::occupancy<P, 16, false, true>(warps, n) : lane::occupancy<P, 16, false, false>(warps, n);
         default: return cudaErrorInvalidValue;
     }
+}
+
+// args of a lane launch: warps per block, the rows they make, traces
+bool args_ok(const SweepArgs &a) {
+    return a.wn >= 1 && a.wn <= lane::kMaxWarps && a.G <= a.seg && a.R == a.wn * (32 / a.seg);
 }
 
 }  // namespace
@@ -120,10 +188,23 @@ bool sweep_lane_supports(int P, int precision, int seg) {
     return P >= 1 && P <= 3 && (precision == 0 || precision == 2) && (seg == 4 || seg == 8 || seg == 16);
 }
 
-int sweep_lane_warps() { return lane::kWarps; }
+// Compute warps per thread block, for a launch of row_blocks(w) items with w warps.  Small launches are bound by the
+// latency of an iteration, and two warps on one SM sub-partition slow each other: 3 warps and the helper (one warp per
+// sub-partition) while every block then has an SM of its own, else 4 likewise; large ones by the warps in flight and the
+// handoffs through L2 between blocks: 7 and the helper.  At DG degree 2, whose iterations keep a sub-partition busier, 4
+// up to 4/3 blocks per SM.  B200, sweep kernel in us with 3 / 4 / 7 warps: 64x64 Q1 S8 66.5 / - / 73.7, 128x128 Q1 S16
+// 159 / 137 / 153, 192x160 Q2 S12 381 / 359 / 378, 256x256 Q1 S12 316 / 323 / 307, 256x256 Q2 S16 691 / - / 671; its
+// moments-only sweep 370 / - / 324.
+int sweep_lane_warps(int P, int seg, bool src2, int num_sms, const std::function<int64_t(int)> &row_blocks) {
+    int w = row_blocks(3) <= num_sms                              ? 3
+            : row_blocks(4) <= (P == 3 ? num_sms * 4 / 3 : num_sms) ? 4
+                                                                    : lane::kMaxWarps;
+    while (w > 1 && lane::block_smem_bytes(P, seg, src2, false, w) > (size_t)(224 << 10)) --w;
+    return w;
+}
 
 cudaError_t launch_sweep_lane(int P, int precision, const SweepArgs &args, int grid, cudaStream_t stream) {
-    if (!args.trace || args.G > args.seg || args.R != 32 / args.seg) return cudaErrorInvalidValue;
+    if (!args.trace || !args_ok(args)) return cudaErrorInvalidValue;
     if (precision != 0 && precision != 2) return cudaErrorInvalidValue;
     const bool fp32 = precision == 2;
     switch (P) {
@@ -134,77 +215,107 @@ cudaError_t launch_sweep_lane(int P, int precision, const SweepArgs &args, int g
     }
 }
 
-cudaError_t launch_modal_sources(const GridDims &g, const double *moments, double scale, double *out, cudaStream_t s) {
-    const size_t n = (size_t)g.nx * g.ny * 4;
+cudaError_t launch_modal_sources(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
+                                 double scale, bool adjoint, double *out, cudaStream_t s) {
+    const int b = blocks_for((size_t)g.nx * g.ny * 4);
+    switch (g.P + (adjoint ? 4 : 0)) {
+        case 1: modal_sources_kernel<1, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 2: modal_sources_kernel<2, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 3: modal_sources_kernel<3, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 5: modal_sources_kernel<1, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 6: modal_sources_kernel<2, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 7: modal_sources_kernel<3, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cell_records(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
+                                double *out, cudaStream_t s) {
+    const int b = blocks_for((size_t)g.nx * g.ny * cell_record_doubles(g.P));
     switch (g.P) {
-        case 1: modal_sources_kernel<1><<<blocks_for(n), 256, 0, s>>>(g, moments, scale, out); break;
-        case 2: modal_sources_kernel<2><<<blocks_for(n), 256, 0, s>>>(g, moments, scale, out); break;
-        case 3: modal_sources_kernel<3><<<blocks_for(n), 256, 0, s>>>(g, moments, scale, out); break;
+        case 1: cell_records_kernel<1><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
+        case 2: cell_records_kernel<2><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
+        case 3: cell_records_kernel<3><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_modal_partials(const GridDims &g, const double *part, const int slot_begin[5], size_t stride,
-                                         double *phi, cudaStream_t s) {
+                                         bool adjoint, const double *minuend, double *phi, cudaStream_t s) {
     SlotBounds sb;
     for (int k = 0; k < 5; ++k) sb.b[k] = slot_begin[k];
-    const size_t n = (size_t)(g.nx + 2) * (g.ny + 2);
-    switch (g.P) {
-        case 1: reduce_modal_partials_kernel<1><<<blocks_for(n), 256, 0, s>>>(g, part, sb, stride, phi); break;
-        case 2: reduce_modal_partials_kernel<2><<<blocks_for(n), 256, 0, s>>>(g, part, sb, stride, phi); break;
-        case 3: reduce_modal_partials_kernel<3><<<blocks_for(n), 256, 0, s>>>(g, part, sb, stride, phi); break;
+    const int b = blocks_for((size_t)(g.nx + 2) * (g.ny + 2));
+    switch (g.P + (adjoint ? 4 : 0)) {
+        case 1: reduce_modal_partials_kernel<1, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 2: reduce_modal_partials_kernel<2, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 3: reduce_modal_partials_kernel<3, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 5: reduce_modal_partials_kernel<1, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 6: reduce_modal_partials_kernel<2, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 7: reduce_modal_partials_kernel<3, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
 namespace {
-template <int P>
+template <int P, bool PHI>
 cudaError_t launch_batched_p(int seg, const SweepArgs &args, const SweepArgs *table, int grid, cudaStream_t stream) {
     switch (seg) {
-        case 4: return lane::launch_batched<P, 4>(args, table, grid, stream);
-        case 8: return lane::launch_batched<P, 8>(args, table, grid, stream);
-        case 16: return lane::launch_batched<P, 16>(args, table, grid, stream);
+        case 4: return lane::launch_batched<P, 4, PHI>(args, table, grid, stream);
+        case 8: return lane::launch_batched<P, 8, PHI>(args, table, grid, stream);
+        case 16: return lane::launch_batched<P, 16, PHI>(args, table, grid, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 template <int P>
-cudaError_t occupancy_batched_p(int seg, int *n) {
+cudaError_t launch_batched_any(const SweepArgs &args, const SweepArgs *table, int members, bool moments_only, int grid,
+                               cudaStream_t stream) {
+    if (!moments_only) return launch_batched_p<P, false>(args.seg, args, table, grid, stream);
+    const dim3 helpers(148, (unsigned)members);   // grid-stride over each problem's cells
+    modal_sources_batched_kernel<P><<<helpers, 256, 0, stream>>>(table);
+    cudaError_t e = launch_batched_p<P, true>(args.seg, args, table, grid, stream);
+    if (e != cudaSuccess) return e;
+    reduce_modal_batched_kernel<P><<<helpers, 256, 0, stream>>>(table);
+    return cudaGetLastError();
+}
+template <int P>
+cudaError_t occupancy_batched_p(int seg, int warps, int *n) {
     switch (seg) {
-        case 4: return lane::occupancy_batched<P, 4>(n);
-        case 8: return lane::occupancy_batched<P, 8>(n);
-        case 16: return lane::occupancy_batched<P, 16>(n);
+        case 4: return lane::occupancy_batched<P, 4>(warps, n);
+        case 8: return lane::occupancy_batched<P, 8>(warps, n);
+        case 16: return lane::occupancy_batched<P, 16>(warps, n);
         default: return cudaErrorInvalidValue;
     }
 }
 }  // namespace
 
-cudaError_t launch_sweep_lane_batched(int P, const SweepArgs &args, const SweepArgs *table, int grid,
-                                      cudaStream_t stream) {
-    if (args.G > args.seg || args.R != 32 / args.seg || !table) return cudaErrorInvalidValue;
+cudaError_t launch_sweep_lane_batched(int P, const SweepArgs &args, const SweepArgs *table, int members, bool moments_only,
+                                      int grid, cudaStream_t stream) {
+    if (!args_ok(args) || !table) return cudaErrorInvalidValue;
     switch (P) {
-        case 1: return launch_batched_p<1>(args.seg, args, table, grid, stream);
-        case 2: return launch_batched_p<2>(args.seg, args, table, grid, stream);
-        case 3: return launch_batched_p<3>(args.seg, args, table, grid, stream);
+        case 1: return launch_batched_any<1>(args, table, members, moments_only, grid, stream);
+        case 2: return launch_batched_any<2>(args, table, members, moments_only, grid, stream);
+        case 3: return launch_batched_any<3>(args, table, members, moments_only, grid, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t sweep_lane_batched_occupancy(int P, int seg, int *blocks_per_sm) {
+cudaError_t sweep_lane_batched_occupancy(int P, int seg, int warps, int *blocks_per_sm) {
     switch (P) {
-        case 1: return occupancy_batched_p<1>(seg, blocks_per_sm);
-        case 2: return occupancy_batched_p<2>(seg, blocks_per_sm);
-        case 3: return occupancy_batched_p<3>(seg, blocks_per_sm);
+        case 1: return occupancy_batched_p<1>(seg, warps, blocks_per_sm);
+        case 2: return occupancy_batched_p<2>(seg, warps, blocks_per_sm);
+        case 3: return occupancy_batched_p<3>(seg, warps, blocks_per_sm);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t sweep_lane_occupancy(int P, int seg, bool src2, int *blocks_per_sm) {
+cudaError_t sweep_lane_occupancy(int P, int seg, int warps, bool src2, int *blocks_per_sm) {
     switch (P) {
-        case 1: return occ_p<1>(seg, src2, blocks_per_sm);
-        case 2: return occ_p<2>(seg, src2, blocks_per_sm);
-        case 3: return occ_p<3>(seg, src2, blocks_per_sm);
+        case 1: return occ_p<1>(seg, warps, src2, blocks_per_sm);
+        case 2: return occ_p<2>(seg, warps, src2, blocks_per_sm);
+        case 3: return occ_p<3>(seg, warps, src2, blocks_per_sm);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -5,47 +5,54 @@
 // SweepCellSolveBase::ConstructAndSolve (linear_solvers/RKDG/SweepCellSolve/SweepCellSolve.hpp:312-353),
 // in the packed modal basis of modal_cell.cuh (the same cell arithmetic as sweep_modal_impl.cuh).
 //
-// Every warp is an independent worker with its own work item: Rw = 32/SEG consecutive rows (in sweep
-// order) of one quadrant for one chunk of <= SEG ordinates, swept across all columns.  Lane (rr, o) =
-// (lane / SEG, lane % SEG) owns ordinate q_begin + o on row rr; row rr runs one column behind row rr-1 and
-// takes its y trace by __shfl_up, the x trace stays in the lane.  Iteration s of a warp does, for every
-// lane, the work of three cells:
-//   * the chain of step s: the y trace in, the modal cell step, the traces out (the only dependency from
-//     cell to cell, so the only part whose latency sits on the wavefront's critical path);
-//   * the finish of step s - 1: the backward transform; psi through a per-warp shared buffer whose rows are
-//     the reference's contiguous row segments, one bulk copy (cp.async.bulk) per row segment; the row
-//     segment's moment sums (a shuffle butterfly for 4- and 8-wide segments, sums over a k-major shared
-//     buffer for 16-wide ones), one partial per ordinate chunk, each a fixed tree, added in a fixed order by
-//     reduce_phi_partials: bitwise reproducible;
-//   * the inputs of step s + 1: the forward modal transform and the reciprocal denominators of its source
-//     dofs and sigma_t (and second source, and fused scattering moments), which were copied into shared
-//     memory by cp.async kStages - 2 iterations earlier.
-// After the y trace's arrival (and, rarely, a wait for the producer) the chain, the finish and the transform
-// are one basic block with the chain first: every global access in it is predicated instead of branched
-// around, so the scheduler interleaves the three cells' instructions.  The loads and copies for later steps
-// and the work behind uniform branches (scattering moments, psi rows that are not 16-byte aligned) follow in
-// a tail section.  Measured on B200 at 256x256 Q2 S16 (FP64): the branchy form of the same work ran its
-// phases one after another (the per-phase times summed to the iteration time) and scattered 8-byte psi
-// stores, 32 sectors per instruction, were a third of the kernel's time.  The loop body is one iteration for
-// every quadrant (the quadrant's sign flips are applied to the cell values at run time as sign-bit flips,
-// exact), so the hot loop stays small for the instruction caches.  Four warps per thread block, one per SM
-// sub-partition.
+// An item is a group of consecutive row blocks of one quadrant for one chunk of <= SEG ordinates, swept across all
+// columns by one thread block: warp w owns row block w of the group, Rw = 32/SEG rows (in sweep order).  Lane (rr, o) =
+// (lane / SEG, lane % SEG) owns ordinate q_begin + o on row rr; row rr runs one column behind row rr-1 and takes its y
+// trace by __shfl_up, the x trace stays in the lane.  A block's last warp is its helper: it takes the block's items from
+// the queue and feeds the traces of the row above the block to the first warp.
 //
-// Between row blocks: the warp's last row writes its outgoing y traces, column by column, into the item's
-// trace buffer with relaxed 8-byte stores; row 0 of the item below loads column s + 1 with relaxed loads at
-// iteration s.  A value still holding the NaN-payload sentinel means the consumer has caught up with its
-// producer: it then polls (bounded) until the producer has written that column, and no further, which
-// keeps the lag between row blocks at its minimum.  The consumer writes the sentinel back after use.  The
-// first row block reads the ghost row's inflow traces (inflow_traces_kernel) the same way.  Items are
-// dequeued per warp in row-block order from an atomic counter, so an item's producer is always held by a
-// running warp: no deadlock, and no thread block needs any other to be resident.  Every wait is bounded
-// (spin_limit); on expiry the warp records kDevTimeout in the device error word and leaves, and every other
-// warp leaves when it sees the word.
+// Iteration s of a warp is one basic block after the (rarely taken) waits:
+//   * the chain of step s: the y trace in, the modal cell step, the traces out (the only dependency from cell to cell,
+//     so the only part whose latency sits on the wavefront's critical path); beside it the forward modal transform and
+//     the reciprocal denominators of step s + 1's inputs, copied into shared memory by cp.async kStages - 1 iterations
+//     earlier;
+//   * the finish of step s: the backward transform; psi (degree 2: through a per-warp shared buffer, 16-byte stores of
+//     the row segment's chunks; degree 1: a lane's 32-byte block in one store); the row segment's moment sums (a shuffle
+//     butterfly for 4- and 8-wide segments, sums over a k-major shared buffer for 16-wide ones), one partial per ordinate
+//     chunk, each a fixed tree, added in a fixed order by reduce_phi_partials: bitwise reproducible;
+//   * the copies of step s + kStages.
+// Every global access is predicated instead of branched around, so the scheduler interleaves the parts.  The quadrant's
+// sign flips are applied to the cell values at run time as sign-bit flips (exact): one loop body for every quadrant.
+//
+// What bounds it: a sweep of nx columns and ny rows is nx + ny iterations long plus the handoffs between row blocks, so
+// the time of one iteration of a lone warp (latency, at few warps per sub-partition) and the handoffs set the small
+// sizes, issue slots the large ones.  Measured on B200 (sweep kernel, before -> after each):
+//   * handoff through shared memory, L2 only between blocks and there by the helper: when every warp read the trace of
+//     the row above from L2 itself, no iteration could be shorter than an L2 load (0.56 us at degree 0, where it is 0.2
+//     us of work).  With the rest below, 300x200 Q0 S16 349 -> 202 us, 64x64 Q1 S8 85 -> 66 us, 512x512 Q1 S12 932 -> 753
+//     us; 256x256 Q2 S16 (684 -> 671 us) is bound by issue: 648 warp instructions per iteration, 215 of them FP64, with
+//     255 registers and so two warps per sub-partition.
+//   * psi stores: bulk copies through shared memory (proxy fence, commit, wait) cost 0.25 us an iteration at degree 1;
+//     a lane's own 32-byte store 0.001 (2048x4 Q1 S8, one row block: 1342 -> 832 us).  Degree 2: 16-byte chunks.
+//   * the moments-only sweeps' inputs (modal source and sigma_t) as one record per cell copied once per row, where every
+//     lane had copied its own: 256x256 Q2 S16 566 -> 324 us with the above, 128x128 Q1 S8 117 -> 93 us.
+//   * the backward transform in its own iteration instead of beside the next one's chain: 38 fewer live registers, no
+//     spills at degree 2 (2048x2 Q2 S16, one row block: 1766 -> 1460 us).
+//
+// Handoffs.  Traces travel as 8-byte values that are their own flags: a slot holds a NaN-payload sentinel until its value
+// is written, and the reader writes the sentinel back.  Between the warps of a block a ring of kRing columns in shared
+// memory (the reader publishes how many columns it has read, every fourth column; the writer waits for room); from a
+// block's last warp the item's row of the global trace buffer, relaxed 8-byte stores, which the helper of the block below
+// reads kFeedAhead columns at a time and passes into its first warp's ring.  The grid's first row takes the ghost row's
+// inflow traces (inflow_traces_kernel) the same way.  Items are dequeued in row-group order from an atomic counter, so an
+// item's producer is always held by a running block: no deadlock, and no block needs any other to be resident.  Every
+// wait is bounded (spin_limit); on expiry the warp records kDevTimeout in the device error word and leaves, and every
+// other warp leaves when it sees the word.
 //
 // Transposed sweep (ADJ): reverse traversal order per quadrant, the transposed cell operator and coupling
 // of modal_cell.cuh, zero inflow, the fused source w_q * mu and unweighted moment sums (the transposes of
 // Smv's broadcast and of Pmv).  SRC2 adds a second source, fma(src2_scale, src2, src), as the IDC source
-// kernel combines them.  PHI: the moments-only forward sweep of the Krylov iterations (no source array,
+// kernel combines them.  PHI: the moments-only sweep of the Krylov iterations (no source array,
 // psi not stored): the cell's source is its isotropic scattering source, the same for every ordinate of a
 // quadrant, read already in the packed modal basis (launch_modal_sources, once per cell and quadrant), and
 // the moments are summed in the packed basis (launch_reduce_modal_partials transforms each quadrant's sum
@@ -63,35 +70,38 @@
 namespace idc {
 namespace lane {
 
-constexpr int kWarps = 4;    // warps per thread block: one per SM sub-partition
-constexpr int kStages = 6;   // stages in shared memory: a step's inputs are copied this many steps minus one ahead
-constexpr int kOutBufs = 2;  // psi leaves through a ring of this many per-warp buffers
-constexpr int kMomStride = 34;   // doubles per moment index k in the moment buffer (32 lanes + 2: conflict-free sums)
-// Polls per round of the producer wait below, by DG degree + 1, chosen by measurement on B200 (interleaved
-// A/B).  At DG degree 1 the three-poll form is 6-8% faster (512x512 Q1 S12 1.015-1.039 -> 0.950 ms; two: no
-// gain).  ptxas places its poll array in local memory (a 48-byte stack frame), so its loads do not stay in
-// flight together as the loop is written; variants with the polls in registers (overlapping), with one poll
-// and a 256 ns sleep, or waiting for 2 or 4 columns of slack all lose the gain (1.02-1.18 ms), so where the
-// gain comes from is not established.  At DG degree 2 three polls cost 2-3% (0.695 -> 0.714 ms): one.
-template <int P>
-constexpr int kPollDepth = P >= 3 ? 1 : 3;
+constexpr int kMaxWarps = 7;   // compute warps per thread block; the helper warp is the eighth (two per SM sub-partition)
+constexpr int kStages = 6;     // stages in shared memory: a step's inputs are copied this many steps minus one ahead
+constexpr int kRing = 8;       // columns of y traces between two warps of a thread block
+constexpr int kMomStride = 34; // doubles per moment index k in the moment buffer (32 lanes + 2: conflict-free sums)
 
-// Doubles per (column, ordinate) slot of the trace buffer.
-__host__ __device__ constexpr int trace_slot(int P) { return P; }
+// Degrees 1 and 2 copy a row segment's source dofs to shared memory, and degree 2 its psi back, in 16-byte chunks: lane o
+// of the row takes chunks o, o + SEG, ... of the segment, whose start is moved down to a 16-byte boundary (copies are
+// coalesced whatever the degree, where a lane's own 72-byte block at degree 2 would take nine 8-byte accesses in as many
+// sectors).  Chunks per lane, and doubles from one row's block in shared memory to the next (it starts at the parity, in
+// 8-byte words, of its global address).
+__host__ __device__ constexpr bool chunked(int P) { return P >= 2; }
+__host__ __device__ constexpr int lane_chunks(int P, int seg) { return (seg * P * P / 2 + 1 + seg - 1) / seg; }
+__host__ __device__ constexpr int row_pitch(int P, int seg) { return chunked(P) ? 2 * seg * lane_chunks(P, seg) + 2 : seg; }
 
-// Shared memory of one warp, in doubles: source stages [kStages][32][N] (lane-major, conflict-free), the
-// second source's stages (launches with one), sigma_t stages [kStages][32] (each lane its own copy), the
-// fused scattering moments' stages [kStages][Rw][N] (copied by lane o == 0 of each row) and the psi out
-// buffers [kOutBufs][32][N] (lane-major: row rr's SEG ordinates are the reference's contiguous row segment)
-// and, for 16-wide segments, the weighted moment values [N][kMomStride] (k-major: a row segment's SEG values
-// of one k are adjacent).
-// Every part is an even number of doubles, so each starts on a 16-byte boundary.
-__host__ __device__ constexpr size_t warp_doubles(int P, int seg, bool src2) {
-    return (size_t)kStages * 32 * P * P * (src2 ? 2 : 1) + (size_t)kStages * 32 + (size_t)kStages * (32 / seg) * P * P +
-           (size_t)kOutBufs * 32 * P * P + (seg >= 16 ? (size_t)P * P * kMomStride : 0);
+// Shared memory of one warp, in doubles (every part an even number, so each starts on a 16-byte boundary): source
+// stages [kStages][Rw][pitch], the second source's, cell records [kStages][Rw][cell_record_doubles] (sigma_t and the
+// scattering moments, one copy per row), at degree 2 the psi out buffer [Rw][pitch] and, for 16-wide segments, the
+// weighted moment values [N][kMomStride] (k-major: a row segment's values of one k are adjacent).
+__host__ __device__ constexpr size_t warp_doubles(int P, int seg, bool src2, bool phi) {
+    return (size_t)kStages * (32 / seg) * row_pitch(P, seg) * (phi ? 0 : src2 ? 2 : 1) +
+           (size_t)kStages * (32 / seg) * cell_record_doubles(P) +
+           (phi || P < 3 ? 0 : (size_t)(32 / seg) * row_pitch(P, seg)) +
+           (seg >= 16 ? (size_t)P * P * kMomStride : 0);
 }
-__host__ __device__ constexpr size_t block_smem_bytes(int P, int seg, bool src2) {
-    return sizeof(double) * warp_doubles(P, seg, src2) * kWarps;
+// Doubles of one warp's trace ring [kRing][seg][P].
+__host__ __device__ constexpr size_t ring_doubles(int P, int seg) { return (size_t)kRing * seg * P; }
+// Doubles of the block's common part: the zero source of lanes without one and the consumed-column counts of every warp.
+__host__ __device__ constexpr size_t common_doubles(int P, int warps) {
+    return (size_t)((P * P + 1) / 2 * 2) + (size_t)((warps + 3) / 4 * 2);
+}
+__host__ __device__ constexpr size_t block_smem_bytes(int P, int seg, bool src2, bool phi, int warps) {
+    return sizeof(double) * (warps * (warp_doubles(P, seg, src2, phi) + ring_doubles(P, seg)) + common_doubles(P, warps));
 }
 
 // x with its sign bit flipped where `mask` has it (mask: 0 or 0x80000000, the sign bit of a float or of a
@@ -145,187 +155,220 @@ __device__ __forceinline__ double ld_relaxed_f64_if(const double *p, bool pred) 
                  : "l"(p), "r"((int)pred));
     return v;
 }
-// 8-byte cp.async that writes zeros into dst where the predicate is false (source size 0: nothing is read;
-// callers still pass a source inside a valid allocation)
-__device__ __forceinline__ void cp_async8_zfill(void *dst, const void *src, bool pred) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(saddr(dst)), "l"(src), "r"(pred ? 8 : 0));
-}
-// 16-byte cp.async (through L2) with the same zero fill; dst and src 16-byte aligned
-__device__ __forceinline__ void cp_async16_zfill(void *dst, const void *src, bool pred) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst)), "l"(src), "r"(pred ? 16 : 0));
-}
-// n doubles (n even: 16-byte copies when `wide`, both addresses then 16-byte aligned; else 8-byte copies)
-template <int n>
-__device__ __forceinline__ void cp_async_doubles(double *dst, const double *src, bool pred, bool wide) {
-    if constexpr (n % 2 == 0) {
-        if (wide) {
-#pragma unroll
-            for (int h = 0; h < n / 2; ++h) cp_async16_zfill(dst + 2 * h, src + 2 * h, pred);
-            return;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < n; ++k) cp_async8_zfill(dst + k, src + k, pred);
-}
 __device__ __forceinline__ void cp_async8_if(void *dst, const void *src, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q cp.async.ca.shared.global [%0], [%1], 8;\n\t}" ::"r"(
                      saddr(dst)),
                  "l"(src), "r"((int)pred));
 }
 
-// Bulk copies shared -> global (the copy engine reads the buffer after the issuing thread moves on): one
-// per row segment of psi.  The writes into the buffer are made visible to the copy engine by the proxy fence.
-__device__ __forceinline__ void bulk_store_if(double *dst, const double *src, unsigned bytes, bool pred) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t@q cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\t}" ::"l"(dst),
-                 "r"(saddr(src)), "r"(bytes), "r"((int)pred)
+__device__ __forceinline__ void cp_async16_if(void *dst, const void *src, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(
+                     saddr(dst)),
+                 "l"(src), "r"((int)pred));
+}
+// Trace rings in shared memory: 8-byte values that are their own flags (relaxed within the block), and the count of
+// columns a ring's consumer has read and re-armed (release / acquire).
+__device__ __forceinline__ double ld_ring_if(uint32_t p, bool pred) {   // 0.0 where the predicate is false
+    double v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+                 "@q ld.relaxed.cta.shared::cta.f64 %0, [%1];\n\t}"
+                 : "=d"(v)
+                 : "r"(p), "r"((int)pred));
+    return v;
+}
+__device__ __forceinline__ void st_ring_if(uint32_t p, double v, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.relaxed.cta.shared::cta.f64 [%0], %1;\n\t}" ::"r"(p),
+                 "d"(v), "r"((int)pred));
+}
+// a trace value out: into the next warp's ring or the trace buffer (a generic address)
+__device__ __forceinline__ void st_trace_if(double *p, double v, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.relaxed.gpu.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+                 "r"((int)pred));
+}
+__device__ __forceinline__ int ld_consumed(uint32_t p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_consumed_if(uint32_t p, int v, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.release.cta.shared::cta.s32 [%0], %1;\n\t}" ::"r"(p),
+                 "r"(v), "r"((int)pred)
                  : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int n>
-__device__ __forceinline__ void bulk_wait_read() {
-    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(n) : "memory");
-}
-template <int n>
-__device__ __forceinline__ void bulk_wait() {
-    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(n) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// The consumer caught up with its producer (a value of column s still held the sentinel): wait, bounded,
-// until the producer has written column s.  Waiting for no more than that keeps the lag between row blocks
-// at its minimum (measured on B200: waiting for two more columns of slack, to wait less often, made the
-// 256x256 Q2 S16 sweep 10-20% slower).  The poll that finds the column complete has read its values, which
-// are returned with the poll count, so the consumer does not load them again (one L2 round trip less on the
-// row-block handoff); polls = -1 if the wait gave up or another warp has failed (the error word is then
-// set).  Out of line: the hot loop stays small; every argument is a register.
+__device__ __forceinline__ void st_f64x2_if(double *p, double2 v, bool pred) {   // 16-byte aligned
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %3, 0;\n\t@q st.global.v2.f64 [%0], {%1, %2};\n\t}" ::"l"(p), "d"(v.x),
+                 "d"(v.y), "r"((int)pred));
+}
+__device__ __forceinline__ void st_f64x4_if(double *p, double a, double b, double c, double d, bool pred) {   // 32-byte aligned
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q st.global.v4.f64 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(p),
+                 "d"(a), "d"(b), "d"(c), "d"(d), "r"((int)pred));
+}
+
+// Waits of the hot loop, out of line and bounded: a warp whose wait gives up, or that hears of another's failure,
+// leaves with the error word set.
+constexpr int kReadsPerPoll = 32;     // a poll of the waits on shared memory: this many reads (about 1 us)
+
+// One more poll of a wait: false if it gives up (then the error word is set) or another warp has failed.
+__device__ __forceinline__ bool poll_on(long long &polls, int *error, long long spin_limit, int lane) {
+    if (++polls > spin_limit) {
+        if (lane == 0) atomicCAS(error, kDevOk, kDevTimeout);
+        return false;
+    }
+    int e = 0;
+    if ((polls & 15) == 0 && lane == 0) e = ld_relaxed(error);
+    return __shfl_sync(kFullMask, e, 0) == kDevOk;
+}
+// The ring whose consumer has read `*consumed` columns has no room for `column`: wait, and return the first column
+// that may not be written yet, or -1.
+__device__ __forceinline__ int wait_for_credit(uint32_t consumed, int column, int *error, long long spin_limit, int lane) {
+    for (long long polls = 0;;) {
+        for (int k = 0; k < kReadsPerPoll; ++k) {
+            int c = 0;
+            if (lane == 0) c = ld_consumed(consumed);
+            c = __shfl_sync(kFullMask, c, 0);
+            if (column < c + kRing) return c + kRing;
+            __nanosleep(200);
+        }
+        if (!poll_on(polls, error, spin_limit, lane)) return -1;
+    }
+}
+// Something step s needs is not there: its column of the ring above (not written yet), or room for column cout in the ring
+// below.  Waits for both.
 template <int P>
-struct ProducerWait {
-    long long polls;
-    double v[P];   // column s as the last poll read it; 0.0 in lanes that do not read (as load_trace gives)
+struct StepWait {
+    double v[P];   // the column's traces; 0.0 in lanes that do not read
+    int credit;    // as wait_for_credit; -1: gave up
 };
 template <int P>
-__device__ __noinline__ ProducerWait<P> wait_for_producer(const double *dep_trace, int s, bool reader, int G,
-                                                          int *error, long long spin_limit, long long polls,
-                                                          int lane) {
-    const double *col = dep_trace + (size_t)s * G * P;
-    ProducerWait<P> r;
-    // kPollDepth<P> polls per round: each checked poll is reissued at once
-    double v[kPollDepth<P>][P];
-#pragma unroll
-    for (int d = 0; d < kPollDepth<P>; ++d)
-#pragma unroll
-        for (int m = 0; m < P; ++m) v[d][m] = ld_relaxed_f64_if(col + m, reader);
-    for (;;) {
-#pragma unroll
-        for (int d = 0; d < kPollDepth<P>; ++d) {
+__device__ __noinline__ StepWait<P> wait_for_step(uint32_t slot, bool reader, uint32_t consumed, int cout, int credit,
+                                                  int nx, int *error, long long spin_limit, int lane) {
+    StepWait<P> r;
+    r.credit = -1;
+    for (long long polls = 0;;) {
+        bool there = false;
+        for (int k = 0; k < kReadsPerPoll && !there; ++k) {
             bool still = false;
 #pragma unroll
-            for (int m = 0; m < P; ++m) still |= reader && is_sentinel(v[d][m]);
-            r.polls = polls;
-            if (!__any_sync(kFullMask, still)) {
+            for (int m = 0; m < P; ++m) {
+                r.v[m] = ld_ring_if(slot + 8u * m, reader);
+                still |= reader && is_sentinel(r.v[m]);
+            }
+            there = !__any_sync(kFullMask, still);
+        }
+        if (there) break;
+        if (!poll_on(polls, error, spin_limit, lane)) return r;
+    }
+    if (cout >= credit && cout < nx) {
+        credit = wait_for_credit(consumed, cout, error, spin_limit, lane);
+        if (credit < 0) return r;
+    }
+    r.credit = credit;
+    return r;
+}
+
+// The helper warp: column by column, the traces entering the block's first row (the trace buffer of the item above,
+// polled until its last row has written them and re-armed behind, or the ghost row's inflow) into the first warp's
+// ring.  kFeedAhead columns are loaded at a time, so that the L2 round trip of a load is paid once for as many columns
+// as are there.
+constexpr int kFeedAhead = 4;
+template <int P, int SEG>
+__device__ __forceinline__ void feed_ring(const SweepArgs &a, const SweepItem &item, uint32_t ring, uint32_t consumed,
+                                          int lane) {
+    constexpr int V = SEG * P, NL = (V + 31) / 32;   // values per column, loads per lane and column
+    const bool has_dep = item.dep >= 0;
+    const int count = item.q_count * P;
+    const size_t stride = has_dep ? (size_t)a.G * P : (size_t)a.nq * P;
+    double *src = has_dep ? a.trace + (size_t)item.dep * a.trace_stride
+                          : const_cast<double *>(a.inflow) + (size_t)item.q_begin * P;
+    long long polls = 0;
+    int credit = kRing;
+    int c = 0;
+    while (c < a.nx) {
+        double v[kFeedAhead][NL];
 #pragma unroll
-                for (int m = 0; m < P; ++m) r.v[m] = v[d][m];
-                return r;
-            }
-            ++polls;
-            if ((polls & 63) == 63 && ld_relaxed(error) != kDevOk) {
-                r.polls = -1;
-                return r;
-            }
-            if (polls > spin_limit) {
-                if (lane == 0) atomicCAS(error, kDevOk, kDevTimeout);
-                r.polls = -1;
-                return r;
-            }
+        for (int k = 0; k < kFeedAhead; ++k)
 #pragma unroll
-            for (int m = 0; m < P; ++m) v[d][m] = ld_relaxed_f64_if(col + m, reader);
+            for (int h = 0; h < NL; ++h)
+                v[k][h] = ld_relaxed_f64_if(src + (size_t)(c + k) * stride + lane + 32 * h,
+                                            c + k < a.nx && lane + 32 * h < count);
+        int done = 0;
+        bool go = true;
+#pragma unroll
+        for (int k = 0; k < kFeedAhead; ++k) {
+            if (go && c + k < a.nx) {
+                bool still = false;
+#pragma unroll
+                for (int h = 0; h < NL; ++h) still |= lane + 32 * h < count && is_sentinel(v[k][h]);
+                if (has_dep && __any_sync(kFullMask, still)) {
+                    go = false;
+                } else {
+                    if (c + k >= credit) {
+                        credit = wait_for_credit(consumed, c + k, a.error, a.spin_limit, lane);
+                        if (credit < 0) return;
+                    }
+                    const uint32_t slot = ring + 8u * (uint32_t)(((c + k) % kRing) * V + lane);
+#pragma unroll
+                    for (int h = 0; h < NL; ++h) {
+                        const bool p = lane + 32 * h < count;
+                        st_ring_if(slot + 256u * h, v[k][h], p);
+                        st_relaxed_f64_if(src + (size_t)(c + k) * stride + lane + 32 * h, sentinel_value(), p && has_dep);
+                    }
+                    ++done;
+                }
+            }
+        }
+        c += done;
+        if (done == 0) {
+            if (!poll_on(polls, a.error, a.spin_limit, lane)) return;
+        } else {
+            polls = 0;
         }
     }
 }
 
-// The backward transform of one cell, x = Vb Z Vb^T, and the forward transform of another, S = Wb v Wb^T
-// (modal_backward and modal_forward of modal_cell.cuh with no flips: the same operations in the same order,
-// so the results are bitwise theirs), emitted statement by statement side by side: the two independent FMA
-// chains are adjacent in the instruction stream, and each FMA of one can issue while the other's previous
-// result is still in the pipe.
-template <int P, typename T, bool ADJ>
-__device__ __forceinline__ void modal_backward_forward(T (&x)[P * P], const T (&Z)[P * P], T (&S)[P * P],
-                                                       const T (&v)[P * P]) {
-    T tb[P * P], tf[P * P];
-#pragma unroll
-    for (int i = 0; i < P; ++i)
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            // backward: tb(d = i, b = k) = sum_a Vb(d,a) Z(a,b); forward: tf(a = i, e = k) = sum_d Wb(a,d) v(d,e)
-            T ab = Z[k] * T(basis_v<P, ADJ>(i, 0));
-            T af = v[k] * T(basis_w<P, ADJ>(i, 0));
-#pragma unroll
-            for (int m = 1; m < P; ++m) {
-                ab = fma(T(basis_v<P, ADJ>(i, m)), Z[k + P * m], ab);
-                af = fma(T(basis_w<P, ADJ>(i, m)), v[k + P * m], af);
-            }
-            tb[k + P * i] = ab;
-            tf[k + P * i] = af;
-        }
-#pragma unroll
-    for (int i = 0; i < P; ++i)
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            // backward: x(d = i, e = k) = sum_b Vb(e,b) tb(d,b); forward: S(a = i, b = k) = sum_e Wb(b,e) tf(a,e)
-            T ab = tb[P * i] * T(basis_v<P, ADJ>(k, 0));
-            T af = tf[P * i] * T(basis_w<P, ADJ>(k, 0));
-#pragma unroll
-            for (int m = 1; m < P; ++m) {
-                ab = fma(T(basis_v<P, ADJ>(k, m)), tb[m + P * i], ab);
-                af = fma(T(basis_w<P, ADJ>(k, m)), tf[m + P * i], af);
-            }
-            x[k + P * i] = ab;
-            S[k + P * i] = af;
-        }
-}
-
+// One warp's part of an item: its Rw rows across all columns.  ring_in: the ring (shared address) that feeds its first
+// row if `fed` (else that row's y traces are zero: the grid's first row without inflow); ring_out: the next warp's ring,
+// or null (the warp writes the item's trace buffer); consumed: this ring's count of columns read, the next ring's four
+// bytes on.
 template <int P, int SEG, bool ADJ, bool SRC2, bool PHI, typename TC>
-__device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &item, int it_index, double *wsm,
+__device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &item, int it_index, int row_w, double *wsm,
+                                         const double *zero, uint32_t ring_in, bool fed, double *ring_out, uint32_t consumed,
                                          int lane) {
-    constexpr int N = P * P, Rw = 32 / SEG, D = kStages;
-    if (a.quad_mask != 0 && ((a.quad_mask >> item.quadrant) & 1) == 0) return;   // another quadrant's launch
+    constexpr int N = P * P, Rw = 32 / SEG, D = kStages, V = SEG * P, PITCH = row_pitch(P, SEG);
+    constexpr int RD = cell_record_doubles(P), CH = RD / 2;
+    constexpr int NC = lane_chunks(P, SEG);
+    constexpr bool CHUNK = chunked(P) && !PHI, OBUF = P >= 3 && !PHI;
     // quadrant signs: flips of the cell values (exact), traversal directions (reversed for the transpose)
     const bool XN = item.quadrant >= 2, YN = (item.quadrant & 1) != 0;
     const bool TX = XN != ADJ, TY = YN != ADJ;
     const int quadrant = item.quadrant;
     const int rr = lane / SEG, o = lane - rr * SEG;
-    const int row_w = item.row_block * Rw;
     const int row = row_w + rr;
     const bool row_valid = row < a.ny;
     const bool act = (o < item.q_count) && row_valid;
     const int q = item.q_begin + (act ? o : 0);
-    const int j = row_valid ? (TY ? (a.ny - row) : (1 + row)) : 1;
+    auto row_j = [&](int r) { return TY ? (a.ny - r) : (1 + r); };   // array y index of a sweep row
+    const int j = row_valid ? row_j(row) : 1;
     const int nx = a.nx;
     const size_t plane = (size_t)a.nq * N;
-    const size_t istride = (size_t)(a.ny + 2) * plane;
     const size_t cstride = (size_t)(a.ny + 2);
-    const bool has_dep = item.dep >= 0;
     const bool has_consumer = row_w + Rw < a.ny;
-    const bool has_scatter = !PHI && a.phi_scatter != nullptr;
+    const bool has_rec = PHI || a.cell_rec != nullptr;
+    const bool has_src = !PHI && a.src != nullptr;
     const int T = nx + Rw - 1;
-    const size_t tcol = (size_t)a.G * P;   // doubles per trace column
     const int xi0 = TX ? nx : 1, xis = TX ? -1 : 1;   // array x index of sweep column c: xi0 + xis * c
     const unsigned xm = XN ? 0x80000000u : 0u, ym = YN ? 0x80000000u : 0u;
     auto fmask = [&](int k) { return ((k / P) & 1 ? xm : 0u) ^ ((k % P) & 1 ? ym : 0u); };   // k = e + P d
-    const double *valid_addr = a.sigma_t;   // a source address for accesses that are not made
 
-    double *stage = wsm + (size_t)lane * N;                            // step t at + (t % D) * 32 * N
-    double *stage2 = wsm + (size_t)D * 32 * N + (size_t)lane * N;      // (SRC2 launches only)
-    double *sig = wsm + (size_t)D * 32 * N * (SRC2 ? 2 : 1) + lane;    // + (t % D) * 32
-    double *mom = wsm + (size_t)D * 32 * N * (SRC2 ? 2 : 1) + (size_t)D * 32 + (size_t)rr * N;   // + (t % D) * Rw * N
-    double *obuf = wsm + (size_t)D * 32 * N * (SRC2 ? 2 : 1) + (size_t)D * 32 + (size_t)D * Rw * N;   // + b * 32 * N
-    double *mbuf = obuf + (size_t)kOutBufs * 32 * N;   // [N][kMomStride]
-    // psi rows leave by bulk copies when every row segment starts and ends on a 16-byte boundary
-    const bool bulk_out = a.out != nullptr && ((size_t)a.out & 15) == 0 && ((size_t)a.nq * N) % 2 == 0 &&
-                          ((size_t)item.q_begin * N) % 2 == 0 && ((size_t)item.q_count * N) % 2 == 0;
+    double *stage = wsm;                                                  // step t at + (t % D) * Rw * PITCH
+    double *stage2 = wsm + (PHI ? 0 : (size_t)D * Rw * PITCH);            // (SRC2 launches only)
+    double *recs = stage2 + (SRC2 ? (size_t)D * Rw * PITCH : 0);          // + (t % D) * Rw * RD
+    double *obuf = recs + (size_t)D * Rw * RD + (size_t)rr * PITCH;       // (its row's block)
+    double *mbuf = recs + (size_t)D * Rw * RD + (OBUF ? (size_t)Rw * PITCH : 0);   // [N][kMomStride]
 
-    // an inactive lane runs the cell step of a unit ordinate (finite values) with moment weight zero, so that
-    // the moment sums need no selects
+    // an inactive lane runs the cell step of a unit ordinate on a zero source with moment weight zero (finite
+    // values), so that the moment sums need no selects
     double axd = 1.0, ayd = 1.0, wq = 0.0;
     if (act) {
         axd = fabs(a.xi[q]) / a.dx;
@@ -345,90 +388,126 @@ __device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &it
         for (int m = 0; m < P; ++m) f[m] = TC(in[m]);
     }
 
-    // row 0 reads its y traces from the item above (sentinel-armed) or the ghost row's inflow, the same way
-    const bool reader = rr == 0 && o < item.q_count && row_valid;
-    double *dep_trace = has_dep ? a.trace + (size_t)item.dep * a.trace_stride + (size_t)o * P : nullptr;
-    const double *tin = has_dep ? dep_trace : ((a.inflow && !ADJ) ? a.inflow + (size_t)q * P : nullptr);
-    const size_t tin_col = has_dep ? tcol : (size_t)a.nq * P;
-    const bool tin_ok = reader && tin != nullptr;
-    double *out_trace = a.trace + (size_t)it_index * a.trace_stride + (size_t)o * P;
+    // row 0's y traces come through the ring; the last row's go to the next warp's ring or the trace buffer
+    const bool reader = fed && rr == 0 && o < item.q_count && row_valid;
     const bool writer = has_consumer && rr == Rw - 1 && o < item.q_count;
-    auto load_trace = [&](int c, long long off, double (&v)[P]) {   // off = c * tin_col
-        const bool p = tin_ok && c < nx;
-        const double *ptr = p ? tin + off : valid_addr;
-#pragma unroll
-        for (int m = 0; m < P; ++m) v[m] = ld_relaxed_f64_if(ptr + m, p);
-    };
+    const bool feeds = ring_out != nullptr && has_consumer;
+    ring_in += 8u * (uint32_t)(o * P);
+    // column c's traces go to tout + (c & tmask) * tstride
+    double *tout = (feeds ? ring_out : a.trace + (size_t)it_index * a.trace_stride) + o * P;
+    const int tmask = feeds ? kRing - 1 : -1, tstride = feeds ? V : a.G * P;
+    int credit = feeds ? kRing : nx;   // first column that may not be written yet
 
-    // Column addresses advance by a fixed stride per step: the prefetch of step t reads column t - rr, whose
-    // cell index (xi0 + xis (t - rr)) cstride + j and psi offset are kept running (prefetches come in step order).
+    // Column addresses advance by a fixed stride per step: step t of row r reads column t - r, whose cell index is
+    // (xi0 + xis (t - r)) cstride + j(r); the offsets are kept running (prefetches come in step order).
     const long long dcol = (long long)xis * (long long)cstride;   // cells between consecutive columns
     const long long dsoff = dcol * (long long)plane;              // psi doubles between them
-    long long pf_cidx = ((long long)xi0 - (long long)xis * rr) * (long long)cstride + j;   // step 0's column
-    long long pf_soff = pf_cidx * (long long)plane + (long long)q * N;
-
-    // step t's inputs into stage slot = t % D, one cp.async group per step; a cell outside the row gets zeros.
-    // With an even number of dofs per cell (DG degree 1) every (cell, ordinate) block starts on a 16-byte
-    // boundary of an aligned array, and the copies are 16 bytes wide (half the copy instructions; measured on
-    // B200 at DG degree 1: see the lane kernel's notes); the stage slots are 16-byte aligned by layout.
-    const bool wide_ok = N % 2 == 0 && ((size_t)valid_addr & 15) == 0;
-    const bool src16 = wide_ok && ((size_t)a.src & 15) == 0;
-    const bool src2_16 = wide_ok && (!SRC2 || ((size_t)a.src2 & 15) == 0);
-    const bool modal16 = wide_ok && (!PHI || ((size_t)a.modal_src & 15) == 0);
-    auto prefetch = [&](int t, int slot) {
-        const int c = t - rr;
-        const bool in = row_valid && c >= 0 && c < nx;
-        const size_t cidx = in ? (size_t)pf_cidx : 0;
-        double *d = stage + (size_t)slot * 32 * N;
-        if constexpr (PHI) {   // the cell's packed modal source of this quadrant (the same for the row segment)
-            const double *g = a.modal_src + (cidx * 4 + quadrant) * N;
-            cp_async_doubles<N>(d, g, in && act, modal16);
-        } else {
-            const bool ps = in && act && a.src != nullptr;
-            const double *g = ps ? a.src + pf_soff : valid_addr;
-            cp_async_doubles<N>(d, g, ps, src16);
-        }
-        if constexpr (SRC2) {
-            double *d2 = stage2 + (size_t)slot * 32 * N;
-            const double *g2 = (in && act) ? a.src2 + pf_soff : valid_addr;
-            cp_async_doubles<N>(d2, g2, in && act, src2_16);
-        }
-        cp_async8_zfill(sig + (size_t)slot * 32, a.sigma_t + cidx, in);
-        if (has_scatter) {   // lane o == 0 of a row copies the cell's fused scattering moments (one copy per row)
-            const bool pm = in && o == 0;
-            const double *gm = pm ? a.phi_scatter + cidx * N : valid_addr;
-            double *dm = mom + (size_t)slot * Rw * N;
+    const long long cell0 = ((long long)xi0 - (long long)xis * rr) * (long long)cstride + j;   // step 0's column
+    const long long seg0 = cell0 * (long long)plane + (long long)item.q_begin * N;             // its row segment
+    long long pf_soff = seg0 + (CHUNK ? 2 * o : (long long)(q - item.q_begin) * N);
+    // parity of a row segment's address in 8-byte words at step t: par ^ (t & podd), kept running (steps s and s + D
+    // share it)
+    static_assert(D % 2 == 0, "steps s and s + D have the same parity");
+    const unsigned podd = (unsigned)dsoff & 1u;
+    unsigned spar = ((unsigned)((size_t)a.src >> 3) + (unsigned)seg0) & 1u;
+    unsigned s2par = SRC2 ? ((unsigned)((size_t)a.src2 >> 3) + (unsigned)seg0) & 1u : 0u;
+    unsigned opar = ((unsigned)((size_t)a.out >> 3) + (unsigned)seg0) & 1u;
+    const int seg_n = item.q_count * N;
+    const bool odd_out = OBUF && a.out != nullptr && (podd | opar | ((unsigned)seg_n & 1u)) != 0;
+    const int out_align = OBUF ? 0 : (int)((size_t)a.out & 31);   // degree 1: 32-byte stores where psi allows
+    // the cell records (or sigma_t alone) of a step's rows are copied once per row: lane l copies chunk l % ch of row
+    // l / ch (16 bytes of the record, or 8 of sigma_t)
+    constexpr int NI = (Rw * CH + 31) / 32;
+    const int ch = has_rec ? CH : 1;
+    const double *rec_src = PHI ? a.modal_src + (size_t)quadrant * RD : has_rec ? a.cell_rec : a.sigma_t;
+    const long long rec_cell = PHI ? 4 * RD : has_rec ? RD : 1;   // doubles per cell
+    int prow[NI], pdst[NI];
+    long long poff[NI];
 #pragma unroll
-            for (int k = 0; k < N; ++k) cp_async8_if(dm + k, gm + k, pm);
+    for (int h = 0; h < NI; ++h) {
+        const int idx = lane + 32 * h;
+        prow[h] = idx / ch;
+        const int k = idx - prow[h] * ch;
+        pdst[h] = prow[h] * RD + (has_rec ? 2 * k : N);
+        if (prow[h] >= Rw || row_w + prow[h] >= a.ny) prow[h] = -(1 << 28);   // nothing to copy: never in range
+        const int r = prow[h] < 0 ? 0 : prow[h];
+        poff[h] = (((long long)xi0 - (long long)xis * r) * (long long)cstride + row_j(row_w + r)) * rec_cell +
+                  (has_rec ? 2 * k : 0);
+    }
+    const long long dpoff = dcol * rec_cell;
+    // step t's inputs into stage slot = t % D; a cell outside the row is not copied (its results are not used)
+    // (par, par2: the sources' parities at step t)
+    auto prefetch = [&](int t, int slot, unsigned par, unsigned par2) {
+        const bool in = row_valid && (unsigned)(t - rr) < (unsigned)nx;
+        if constexpr (CHUNK) {
+            const int lim = in && has_src ? seg_n + (int)par - 2 * o : 0;
+            double *d = stage + (size_t)(slot * Rw + rr) * PITCH + 2 * o;
+            const double *g = a.src + (pf_soff - (long long)par);
+#pragma unroll
+            for (int h = 0; h < NC; ++h) cp_async16_if(d + 2 * SEG * h, g + 2 * SEG * h, lim > 2 * SEG * h);
+            if constexpr (SRC2) {
+                const int lim2 = in ? seg_n + (int)par2 - 2 * o : 0;
+                double *d2 = stage2 + (size_t)(slot * Rw + rr) * PITCH + 2 * o;
+                const double *g2 = a.src2 + (pf_soff - (long long)par2);
+#pragma unroll
+                for (int h = 0; h < NC; ++h) cp_async16_if(d2 + 2 * SEG * h, g2 + 2 * SEG * h, lim2 > 2 * SEG * h);
+            }
+        } else if constexpr (!PHI) {   // degree 0: a row segment's values are adjacent
+            cp_async8_if(stage + (size_t)(slot * Rw + rr) * PITCH + o, a.src + pf_soff, in && act && has_src);
+            if constexpr (SRC2)
+                cp_async8_if(stage2 + (size_t)(slot * Rw + rr) * PITCH + o, a.src2 + pf_soff, in && act);
+        }
+#pragma unroll
+        for (int h = 0; h < NI; ++h) {
+            const bool pr = (unsigned)(t - prow[h]) < (unsigned)nx;
+            double *d = recs + (size_t)slot * Rw * RD + pdst[h];
+            if (has_rec)
+                cp_async16_if(d, rec_src + poff[h], pr);
+            else
+                cp_async8_if(d, rec_src + poff[h], pr);
+            poff[h] += dpoff;
         }
         cp_commit();
-        pf_cidx += dcol;
         pf_soff += dsoff;
     };
-
     // step t's raw inputs from its landed stage: the source (with the second source and the fused scattering
     // source) and sigma_t + 1/dt
-    auto load_inputs = [&](int slot, double (&src)[N], double &st) {   // slot = t % D of step t
-        const double *sp = stage + (size_t)slot * 32 * N;
+    auto load_inputs = [&](int slot, unsigned par, unsigned par2, double (&src)[N], double &st) {   // slot = t % D of step t
+        const double2 *rv = reinterpret_cast<const double2 *>(recs + (size_t)(slot * Rw + rr) * RD);
+        double rp[RD];
+        if (has_rec) {
 #pragma unroll
-        for (int k = 0; k < N; ++k) src[k] = sp[k];
-        if constexpr (SRC2) {
-            const double *sp2 = stage2 + (size_t)slot * 32 * N;
-#pragma unroll
-            for (int k = 0; k < N; ++k) src[k] = fma(a.src2_scale, sp2[k], src[k]);
+            for (int h = 0; h < CH; ++h) {
+                const double2 v = rv[h];
+                rp[2 * h] = v.x;
+                rp[2 * h + 1] = v.y;
+            }
+        } else {
+            rp[N] = recs[(size_t)(slot * Rw + rr) * RD + N];
         }
-        st = sig[(size_t)slot * 32] + a.inv_dt;
-        if (has_scatter) {   // lane o == 0's copy of the cell's moments, handed to its row segment
-            const double *mp = mom + (size_t)slot * Rw * N;
+        if constexpr (PHI) {   // the cell's packed modal source of this quadrant (the transpose's times w_q)
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-                const double mk = __shfl_sync(kFullMask, o == 0 ? mp[k] : 0.0, rr * SEG);
-                if constexpr (!ADJ)   // fused TransportOperator::Smv(scale, 1, sigma_s, phi -> src)
-                    src[k] = fma(a.scatter_scale, mk, src[k]);
-                else                  // the transpose of Pmv: w_q * mu
-                    src[k] = fma(wq, mk, src[k]);
+            for (int k = 0; k < N; ++k) src[k] = ADJ ? wq * rp[k] : rp[k];
+        } else {
+            const double *sp = has_src && act ? stage + (size_t)(slot * Rw + rr) * PITCH + (CHUNK ? par : 0u) + o * N : zero;
+#pragma unroll
+            for (int k = 0; k < N; ++k) src[k] = sp[k];
+            if constexpr (SRC2) {
+                const double *sp2 = act ? stage2 + (size_t)(slot * Rw + rr) * PITCH + (CHUNK ? par2 : 0u) + o * N : zero;
+#pragma unroll
+                for (int k = 0; k < N; ++k) src[k] = fma(a.src2_scale, sp2[k], src[k]);
+            }
+            if (has_rec) {
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    if constexpr (!ADJ)   // fused TransportOperator::Smv(scale, 1, sigma_s, phi -> src)
+                        src[k] = fma(a.scatter_scale, rp[k], src[k]);
+                    else                  // the transpose of Pmv: w_q * mu
+                        src[k] = fma(wq, rp[k], src[k]);
+                }
             }
         }
+        st = rp[N] + a.inv_dt;
     };
     // the modal source and the reciprocal denominators of the raw inputs (the prologue's step; in the loop the
     // forward transform runs beside the previous step's backward transform)
@@ -445,88 +524,70 @@ __device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &it
         }
     };
 
-    // psi of step t from its out buffer (filled at iteration t + 1) with per-lane stores (row segments that are
-    // not 16-byte aligned)
-    auto store_psi_lanes = [&](int t) {
-        const int ct = t - rr;
-        const bool ps = act && ct >= 0 && ct < nx;
-        const double *ob = obuf + (size_t)((t + 1) & (kOutBufs - 1)) * 32 * N + (size_t)lane * N;
-        double *op = ps ? a.out + ((size_t)(xi0 + xis * ct) * cstride + j) * plane + (size_t)q * N : out_trace;
-#pragma unroll
-        for (int k = 0; k < N; ++k) st_f64_if(op + k, ob[k], ps);
-    };
-    const bool lane_out = !PHI && a.out != nullptr && !bulk_out;
-
     const int phi_slot = a.phi_slots > 0 ? it_index % a.phi_slots : 0;
     double *phi_base = a.phi_part ? a.phi_part + (size_t)phi_slot * a.phi_slot_stride : nullptr;
-    long long polls = 0;
 
-    // prologue: stages 0 .. D-1 in flight, step 0 prepared, step 1's raw inputs loaded, row 0's trace of
-    // column 0 loaded
+    // prologue: stages 0 .. D-1 in flight, step 0 prepared
 #pragma unroll
-    for (int t = 0; t < D - 1; ++t) prefetch(t, t);
-    cp_wait<D - 2>();
+    for (int t = 0; t < D; ++t) prefetch(t, t, spar ^ (t & podd), s2par ^ (t & podd));
+    cp_wait<D - 1>();
+    __syncwarp();   // the other lanes' copies
     TC S[N];
     ModalRecip<P, TC> r;
     {
         double src0[N], st0;
-        load_inputs(0, src0, st0);   // slot 0
+        load_inputs(0, spar, s2par, src0, st0);
         transform(src0, st0, S, r);
     }
-    double srcn[N], stn;
-    cp_wait<D - 3>();
-    load_inputs(1, srcn, stn);   // slot 1
-    prefetch(D - 1, D - 1);
+    cp_wait<D - 2>();
+    __syncwarp();
     double tnext[P];
-    load_trace(0, 0, tnext);
-    // per-step running values of the loop: the stage slots of steps s + D (= s % D) and s + 2, the trace column
-    // offsets s * tcol and (s + 1) * tin_col, and the finish column (s - rr - 1)'s cell index and psi offset
-    int sl = 0, sl2 = 2 % D;
-    long long s_tcol = 0, lt_off = (long long)tin_col;
-    const long long out_lag = (long long)(Rw - 1) * (long long)tcol;
-    long long fin_cidx = ((long long)xi0 - (long long)xis * (rr + 1)) * (long long)cstride + j;
-    long long fin_ooff = fin_cidx * (long long)plane + (long long)item.q_begin * N;
-    TC gprev[P], Zp[N];
+#pragma unroll
+    for (int m = 0; m < P; ++m) tnext[m] = ld_ring_if(ring_in + 8u * m, reader);
+    // per-step running values of the loop: the ring slot of column s, the stage slots of steps s and s + 1, and column
+    // s - rr's cell index and psi offset
+    uint32_t ring_slot = ring_in;
+    int sl = 0, sl1 = 1;
+    long long fin_cidx = cell0;
+    long long fin_ooff = seg0;
+    TC gprev[P];
 #pragma unroll
     for (int m = 0; m < P; ++m) gprev[m] = TC(0);
-#pragma unroll
-    for (int k = 0; k < N; ++k) Zp[k] = TC(0);
 
-    // Iteration s: the y trace in (and the wait for a producer, rarely taken); then one basic block with the
-    // chain of step s (s < T) first, as it is the wavefront's critical path, the finish of step s - 1 and the
-    // transform of step s + 1's inputs; then the loads and copies for later steps.
-    for (int s = 0; s <= T; ++s) {
-        const int c = s - rr;
-        const bool valid = act && c >= 0 && c < nx;
+    // Iteration s: the y trace in and the waits (rarely taken); then one basic block: the chain of step s, the
+    // wavefront's critical path, beside the transform of step s + 1's inputs, then step s's backward transform, psi and
+    // moments, and the copies of step s + D.
+    for (int s = 0; s < T; ++s) {
+        const bool inrow = row_valid && (unsigned)(s - rr) < (unsigned)nx;
+        const bool valid = act && inrow;
+        const int cout = s - (Rw - 1);   // the last row's column: its traces go out
 
-        // ---- the y trace in: from the row below (previous step); row 0 from the item above ----
+        // ---- the y trace in: from the row below (previous step); row 0 from the ring ----
         TC g[P];
 #pragma unroll
         for (int m = 0; m < P; ++m) g[m] = __shfl_up_sync(kFullMask, gprev[m], SEG);
-        if (has_dep) {
-            bool bad = false;
+        {
+            const bool p = reader && s < nx;
+            bool wait = cout >= credit && cout < nx;
 #pragma unroll
-            for (int m = 0; m < P; ++m) bad |= reader && s < nx && is_sentinel(tnext[m]);
-            if (__any_sync(kFullMask, bad)) {   // caught up with the producer: wait for column s
-                const ProducerWait<P> w =
-                    wait_for_producer<P>(dep_trace, s, reader, a.G, a.error, a.spin_limit, polls, lane);
-                polls = w.polls;
-                if (polls < 0) break;
+            for (int m = 0; m < P; ++m) wait |= p && is_sentinel(tnext[m]);
+            if (__builtin_expect(__any_sync(kFullMask, wait), 0)) {
+                const StepWait<P> w = wait_for_step<P>(ring_slot, p, consumed + 4u, cout, credit, nx, a.error,
+                                                       a.spin_limit, lane);
+                credit = w.credit;
+                if (credit < 0) break;
 #pragma unroll
                 for (int m = 0; m < P; ++m) tnext[m] = w.v[m];
             }
-        }
-        {   // re-arm the consumed column for the next sweep
-            const bool p = has_dep && reader && s < nx;
-            double *ptr = p ? dep_trace + s_tcol : out_trace;
 #pragma unroll
-            for (int m = 0; m < P; ++m) st_relaxed_f64_if(ptr + m, sentinel_value(), p);
+            for (int m = 0; m < P; ++m) st_ring_if(ring_slot + 8u * m, sentinel_value(), p);   // re-arm
         }
 #pragma unroll
         for (int m = 0; m < P; ++m) g[m] = (rr == 0) ? TC(tnext[m]) : g[m];
-        load_trace(s + 1, lt_off, tnext);
 
-        // ---- the chain of step s ----
+        // ---- the chain of step s, step s + 1's inputs ----
+        double srcn[N], stn;
+        load_inputs(sl1, spar ^ podd, s2par ^ podd, srcn, stn);
         TC Z[N], fn[P], gout[P];
 #pragma unroll
         for (int m = 0; m < P; ++m) fn[m] = f[m];
@@ -534,54 +595,63 @@ __device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &it
 #pragma unroll
         for (int m = 0; m < P; ++m) {
             f[m] = valid ? fn[m] : f[m];
-            gprev[m] = valid ? gout[m] : TC(0);
+            gprev[m] = gout[m];   // the row below uses it for this column: only if the column is one of the row's
         }
-        {   // traces out: relaxed stores, each value its own flag
-            const int cout = s - (Rw - 1);
-            const bool p = writer && cout >= 0 && cout < nx;
-            double *ptr = p ? out_trace + (s_tcol - out_lag) : out_trace;
+        {   // traces out: each value its own flag
+            double *slot = tout + (long long)((cout & tmask) * (long long)tstride);
+            const bool p = writer && (unsigned)cout < (unsigned)nx;
 #pragma unroll
-            for (int m = 0; m < P; ++m) st_relaxed_f64_if(ptr + m, double(gout[m]), p);
+            for (int m = 0; m < P; ++m) st_trace_if(slot + m, double(gout[m]), p);
         }
 
-        // ---- the finish of step s - 1: cell dofs, psi, moments (PHI: the packed modal moments) ----
-        {   // (at s = 0 nothing is valid: Zp is zero and no store is made)
-            const int cp = c - 1;
-            const bool inrow = row_valid && cp >= 0 && cp < nx;
-            const size_t cidx = inrow ? (size_t)fin_cidx : 0;
+        transform(srcn, stn, S, r);   // (step s's are used up)
+
+        // ---- the finish of step s: cell dofs, psi, moments (PHI: the packed modal moments) ----
+        {
             TC x[N];
             if constexpr (PHI) {
 #pragma unroll
-                for (int k = 0; k < N; ++k) x[k] = Zp[k];
-#pragma unroll
-                for (int k = 0; k < N; ++k) S[k] = TC(srcn[k]);
-            } else {   // this step's backward transform beside step s + 1's forward transform
-                TC sv[N];
-#pragma unroll
-                for (int k = 0; k < N; ++k) sv[k] = flip_by(TC(srcn[k]), fmask(k));
-                modal_backward_forward<P, TC, ADJ>(x, Zp, S, sv);
+                for (int k = 0; k < N; ++k) x[k] = Z[k];
+            } else {
+                modal_backward<P, false, false, TC, ADJ>(x, Z);
 #pragma unroll
                 for (int k = 0; k < N; ++k) x[k] = flip_by(x[k], fmask(k));
             }
-            r = modal_recip<P, TC>(od, TC(stn));
-            double *ob = obuf + (size_t)(s & (kOutBufs - 1)) * 32 * N;
-            if constexpr (!PHI) bulk_wait_read<kOutBufs - 1>();   // the copy that read this buffer is done
-            __syncwarp();   // and every lane's reads of the buffers in the previous iterations
-            if constexpr (!PHI) {
+            if constexpr (OBUF || SEG >= 16) __syncwarp();   // every lane's reads of the buffers before
+            if constexpr (OBUF) {
 #pragma unroll
-                for (int k = 0; k < N; ++k) ob[(size_t)lane * N + k] = double(x[k]);
+                for (int k = 0; k < N; ++k) obuf[opar + o * N + k] = double(x[k]);
             }
             if constexpr (SEG >= 16) {
 #pragma unroll
                 for (int k = 0; k < N; ++k) mbuf[k * kMomStride + lane] = double(wv * x[k]);
             }
-            if constexpr (!PHI) fence_proxy_async_smem();
-            __syncwarp();
-            if constexpr (!PHI) {   // row rr's segment: one bulk copy by lane o == 0
-                const bool pb = bulk_out && o == 0 && inrow;
-                double *dst = pb ? a.out + fin_ooff : out_trace;
-                bulk_store_if(dst, ob + (size_t)rr * SEG * N, (unsigned)(item.q_count * N * sizeof(double)), pb);
-                bulk_commit();
+            if constexpr (OBUF || SEG >= 16) __syncwarp();
+            const bool pb = a.out != nullptr && inrow;
+            if constexpr (OBUF) {   // the 16-byte chunks of the row segment
+                const int body = (seg_n - (int)opar) & ~1;
+                const int lim = pb ? body - 2 * o : 0;
+                double *dst = a.out + fin_ooff;
+                const double2 *ov = reinterpret_cast<const double2 *>(obuf + 2 * opar + 2 * o);
+#pragma unroll
+                for (int h = 0; h < NC; ++h) st_f64x2_if(dst + opar + 2 * o + 2 * SEG * h, ov[SEG * h], lim > 2 * SEG * h);
+                if (odd_out) {   // and a first or last double outside them
+                    st_f64_if(dst, double(x[0]), pb && o == 0 && opar != 0);
+                    st_f64_if(dst + seg_n - 1, double(x[N - 1]), pb && o + 1 == item.q_count && (int)opar + body != seg_n);
+                }
+            } else if constexpr (!PHI) {
+                double *dst = a.out + fin_ooff + o * N;
+                if constexpr (N == 4) {   // a lane's block is 32 bytes
+                    if (out_align == 0) {
+                        st_f64x4_if(dst, double(x[0]), double(x[1]), double(x[2]), double(x[3]), pb && act);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < N; ++k) st_f64_if(dst + k, double(x[k]), pb && act);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < N; ++k) st_f64_if(dst + k, double(x[k]), pb && act);
+                }
             }
             // the moments of row rr: sums of the SEG weighted values in fixed trees, one partial per ordinate
             // chunk (added in a fixed order by the reduction kernel: bitwise reproducible).  16-wide segments
@@ -589,7 +659,7 @@ __device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &it
             // sum's 15 dependent adds cost 4% of the 256x256 Q2 S16 sweep on B200); narrower ones by a shuffle
             // butterfly (measured on B200: each is the faster one at its width).
             const bool pp = inrow && phi_base != nullptr;
-            double *pt = pp ? phi_base + cidx * N : out_trace;
+            double *pt = phi_base + fin_cidx * N;
             if constexpr (SEG >= 16) {
                 const int k = o < N ? o : N - 1;
                 const double2 *mv = reinterpret_cast<const double2 *>(mbuf + k * kMomStride + rr * SEG);
@@ -613,56 +683,94 @@ __device__ __forceinline__ void run_item(const SweepArgs &a, const SweepItem &it
                 for (int i = 0; i < (N + SEG - 1) / SEG; ++i) st_f64_if(pt + lo + i, double(x[i]), pp && lo + i < hi);
             }
         }
+        // ---- the copies of step s + D, into the stage of step s (read in the last iteration); step s + 2's inputs ----
+        prefetch(s + D, sl, spar, s2par);
+        cp_wait<D - 2>();
+        __syncwarp();   // the other lanes' copies
+        sl = sl1;
+        sl1 = sl1 + 1 == D ? 0 : sl1 + 1;
+        spar ^= podd;
+        s2par ^= podd;
+        // how far this ring has been read, and its next column
+        st_consumed_if(consumed, s + 1, lane == 0 && (s & 3) == 3);
+        ring_slot = ring_in + 8u * (uint32_t)(((s + 1) & (kRing - 1)) * V);
 #pragma unroll
-        for (int k = 0; k < N; ++k) Zp[k] = Z[k];
-
-
-        // ---- step s + 2's raw inputs (copied D - 2 iterations ago), the copies of step s + D ----
-        if (lane_out) store_psi_lanes(s - 1);
-        cp_wait<D - 3>();
-        load_inputs(sl2, srcn, stn);   // step s + 2
-        prefetch(s + D, sl);           // into the stage of step s (read two iterations ago)
-        sl = sl + 1 == D ? 0 : sl + 1;
-        sl2 = sl2 + 1 == D ? 0 : sl2 + 1;
-        s_tcol += (long long)tcol;
-        lt_off += (long long)tin_col;
+        for (int m = 0; m < P; ++m) tnext[m] = ld_ring_if(ring_slot + 8u * m, reader && s + 1 < nx);
+        opar ^= podd;
         fin_cidx += dcol;
         fin_ooff += dsoff;
     }
     cp_wait<0>();
-    bulk_wait<0>();
 }
 
 // BATCHED: the items of several problems in one launch (a batch's problems of one DG degree, FP64 forward
 // sweeps); each item names its problem in `table` and carries its index within that problem (`local`: its trace
-// row and moment slot, `dep` is local too).  A warp copies its item's entry into shared memory; a problem left
+// row and moment slot, `dep` is local too).  A block copies its item's entry into shared memory; a problem left
 // out of the launch (`skip`) has its items return at once.
 template <int P, int SEG, bool ADJ, bool SRC2, bool PHI, typename TC, bool BATCHED>
-__global__ void __launch_bounds__(kWarps * 32, 1) sweep_lane_kernel(const SweepArgs a,
-                                                                    const SweepArgs *__restrict__ table) {
+__global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
+    sweep_lane_kernel(const SweepArgs a, const SweepArgs *__restrict__ table) {
     static_assert(sizeof(SweepArgs) % 8 == 0, "SweepArgs is copied in 8-byte words");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(16) SweepArgs s_args[BATCHED ? kWarps : 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double *wsm = reinterpret_cast<double *>(smem_raw) + warp_doubles(P, SEG, SRC2) * warp;
-    for (;;) {
-        int it = 0;
-        if (lane == 0) {
-            it = atomicAdd(a.next_item, 1);
-            if (ld_relaxed(a.error) != kDevOk) it = a.n_items;
+    __shared__ __align__(16) SweepArgs s_args;   // (batched launches)
+    __shared__ int s_item;
+    constexpr int N = P * P, Rw = 32 / SEG;
+    constexpr size_t RING = ring_doubles(P, SEG), WD = warp_doubles(P, SEG, SRC2, PHI);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = (int)(blockDim.x >> 5) - 1;
+    double *base = reinterpret_cast<double *>(smem_raw);
+    double *rings = base + (size_t)W * WD;
+    double *zero = rings + (size_t)W * RING;
+    int *consumed = reinterpret_cast<int *>(zero + (N + 1) / 2 * 2);
+    for (int t = threadIdx.x; t < (int)(W * RING); t += blockDim.x) rings[t] = sentinel_value();
+    for (int t = threadIdx.x; t < N; t += blockDim.x) zero[t] = 0.0;
+    __syncthreads();
+    // Both loops meet at two barriers per item: one when every warp is done with the last item, one when the helper
+    // has taken the next.
+    if (warp == W) {
+        for (;;) {
+            __syncthreads();
+            {
+                int it = 0;
+                if (lane == 0) {
+                    it = atomicAdd(a.next_item, 1);
+                    if (ld_relaxed(a.error) != kDevOk || it >= a.n_items) it = -1;
+                    s_item = it;
+                }
+                it = __shfl_sync(kFullMask, it, 0);
+                for (int t = lane; t < W; t += 32) consumed[t] = 0;
+                if (BATCHED && it >= 0) {
+                    const unsigned long long *sw =
+                        reinterpret_cast<const unsigned long long *>(table + a.items[it].problem);
+                    unsigned long long *dw = reinterpret_cast<unsigned long long *>(&s_args);
+                    for (int k = lane; k < (int)(sizeof(SweepArgs) / 8); k += 32) dw[k] = sw[k];
+                }
+            }
+            __syncthreads();
+            const int it = s_item;
+            if (it < 0) return;
+            const SweepItem item = a.items[it];
+            const SweepArgs &b = *(BATCHED ? &s_args : &a);
+            if (BATCHED && b.skip) continue;
+            if (b.quad_mask != 0 && ((b.quad_mask >> item.quadrant) & 1) == 0) continue;
+            if (item.dep >= 0 || (b.inflow && !ADJ)) feed_ring<P, SEG>(b, item, saddr(rings), saddr(consumed), lane);
         }
-        it = __shfl_sync(kFullMask, it, 0);
-        if (it >= a.n_items) return;
-        const SweepItem item = a.items[it];
-        if constexpr (BATCHED) {
-            const unsigned long long *sw = reinterpret_cast<const unsigned long long *>(table + item.problem);
-            unsigned long long *dw = reinterpret_cast<unsigned long long *>(&s_args[warp]);
-            for (int k = lane; k < (int)(sizeof(SweepArgs) / 8); k += 32) dw[k] = sw[k];
-            __syncwarp();
-            if (!s_args[warp].skip) run_item<P, SEG, ADJ, SRC2, PHI, TC>(s_args[warp], item, item.local, wsm, lane);
-            __syncwarp();   // every lane is done with the entry before the next item's copy
-        } else {
-            run_item<P, SEG, ADJ, SRC2, PHI, TC>(a, item, it, wsm, lane);
+    } else {
+        for (;;) {
+            __syncthreads();
+            __syncthreads();
+            const int it = s_item;
+            if (it < 0) return;
+            const SweepItem item = a.items[it];
+            const SweepArgs &b = *(BATCHED ? &s_args : &a);
+            if (BATCHED && b.skip) continue;
+            if (b.quad_mask != 0 && ((b.quad_mask >> item.quadrant) & 1) == 0) continue;   // another quadrant's launch
+            const int row_w = (item.row_block * W + warp) * Rw;
+            if (row_w >= b.ny) continue;
+            const bool fed = warp > 0 || item.dep >= 0 || (b.inflow && !ADJ);
+            run_rows<P, SEG, ADJ, SRC2, PHI, TC>(b, item, BATCHED ? item.local : it, row_w, base + (size_t)warp * WD, zero,
+                                                 saddr(rings + (size_t)warp * RING), fed,
+                                                 warp + 1 < W ? rings + (size_t)(warp + 1) * RING : nullptr,
+                                                 saddr(consumed + warp), lane);
         }
     }
 }
@@ -670,40 +778,42 @@ __global__ void __launch_bounds__(kWarps * 32, 1) sweep_lane_kernel(const SweepA
 template <int P, int SEG, bool ADJ, bool SRC2, bool PHI = false, typename TC = double>
 cudaError_t launch(const SweepArgs &args, int grid, cudaStream_t stream) {
     auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, PHI, TC, false>;
-    const size_t smem = block_smem_bytes(P, SEG, SRC2);
+    const size_t smem = block_smem_bytes(P, SEG, SRC2, PHI, args.wn);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kWarps * 32, smem, stream>>>(args, nullptr);
+    kern<<<grid, (args.wn + 1) * 32, smem, stream>>>(args, nullptr);
     return cudaGetLastError();
 }
 
-// A batch's FP64 forward sweep (items of several problems; `table` on the device, one entry per problem)
-template <int P, int SEG>
+// A batch's FP64 forward sweep, full or moments-only (items of several problems; `table` on the device, one entry per
+// problem)
+template <int P, int SEG, bool PHI>
 cudaError_t launch_batched(const SweepArgs &args, const SweepArgs *table, int grid, cudaStream_t stream) {
-    auto kern = sweep_lane_kernel<P, SEG, false, false, false, double, true>;
-    const size_t smem = block_smem_bytes(P, SEG, false);
+    auto kern = sweep_lane_kernel<P, SEG, false, false, PHI, double, true>;
+    const size_t smem = block_smem_bytes(P, SEG, false, PHI, args.wn);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kWarps * 32, smem, stream>>>(args, table);
+    kern<<<grid, (args.wn + 1) * 32, smem, stream>>>(args, table);
     return cudaGetLastError();
 }
 
+// (of the full sweep: the moments-only instance needs less)
 template <int P, int SEG>
-cudaError_t occupancy_batched(int *blocks_per_sm) {
+cudaError_t occupancy_batched(int warps, int *blocks_per_sm) {
     auto kern = sweep_lane_kernel<P, SEG, false, false, false, double, true>;
-    const size_t smem = block_smem_bytes(P, SEG, false);
+    const size_t smem = block_smem_bytes(P, SEG, false, false, warps);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, kWarps * 32, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, (warps + 1) * 32, smem);
 }
 
 template <int P, int SEG, bool ADJ, bool SRC2>
-cudaError_t occupancy(int *blocks_per_sm) {
+cudaError_t occupancy(int warps, int *blocks_per_sm) {
     auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, false, double, false>;
-    const size_t smem = block_smem_bytes(P, SEG, SRC2);
+    const size_t smem = block_smem_bytes(P, SEG, SRC2, false, warps);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, kWarps * 32, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, (warps + 1) * 32, smem);
 }
 
 }  // namespace lane

@@ -211,9 +211,7 @@ enum { IDC_SCATTER_EXPLICIT = 0, IDC_SCATTER_IMPLICIT = 1 };
  * scattering = IDC_SCATTER_EXPLICIT (IMEX): every substep is one sweep with the scattering lagged to the
  * previous node and corrected by the deferred-correction iterations; with use_graph a step is captured
  * once as a CUDA graph and replayed (lane or modal kernel: DG degree <= 2, piecewise-constant cross
- * sections; at DG degree 1, unless idc_set_tile_shape fixed a shape, a grid too small to give the lane
- * kernel an item for every resident warp runs the step on the modal kernel's (8, 5) shape, the faster one
- * there, and the context's default shape returns afterwards).  Reflecting edges and periodic grids return
+ * sections).  Reflecting edges and periodic grids return
  * IDC_ERR_UNSUPPORTED.  Quadrature sums and residuals are FP64; `precision` selects the
  * sweep arithmetic.  *sweeps receives the number of sweeps performed. */
 int idc_idc_integrate(idc_ctx *ctx, double *psi_inout, const double *source, double dt, int64_t steps,
@@ -233,10 +231,10 @@ int idc_sweep_fused(idc_ctx *ctx, const double *source, double *result, double d
 
 /* Tile shape of the sweep kernel: ordinates per row segment (seg: 4, 8, 16 or 32) and compute warps per
  * thread block.  warps = 0 selects the lane-pipelined kernel (every warp sweeps its own row block of 32/seg
- * rows; seg 4, 8 or 16; FP64 sweeps); warps 1..7 the modal kernel with that many compute warps stacked per
+ * rows and the library picks the warps per thread block; seg 4, 8 or 16; FP64 sweeps); warps 1..7 the modal kernel with that many compute warps stacked per
  * thread block (at most 5 at DG degree 2 and 7 below, fewer if the shape's shared memory would not fit).
  * 0, 0 restores the default (the lane kernel for FP64, the modal kernel for the FP32 modes; 16-wide lane
- * segments at DG degree 2, 8-wide at degree 1 for up to 24 ordinates per quadrant).  The shape applies to sweeps with a source or a psi output; the moments-only
+ * segments at DG degree 2, else the narrowest with the best lane use).  The shape applies to sweeps with a source or a psi output; the moments-only
  * sweeps of the Krylov iterations keep their own default (narrow segments, which suit them).  Results do
  * not depend on it beyond the last bits of the moments. */
 int idc_set_tile_shape(idc_ctx *ctx, int32_t seg, int32_t warps);
