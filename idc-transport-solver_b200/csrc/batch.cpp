@@ -486,7 +486,9 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
             any |= !S[p].done;
         }
         if (!any) break;
-        // the vectors to apply A to: x (a restart's true residual) or the next basis (preconditioned) vector
+        // the vectors to apply A to: x (a restart's true residual) or the next basis (preconditioned) vector; the
+        // members' DSA applications share launches (those with one number of CG steps)
+        std::map<int, std::vector<DsaJob>> dsa;
         for (size_t p = 0; p < M; ++p) {
             State &z = S[p];
             if (z.done) continue;
@@ -494,9 +496,11 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
             z.in = z.restart_pending ? z.x : z.dsa ? z.Zc(z.j) : z.Vc(z.j);
             z.out = z.restart_pending ? z.Vc(0) : z.Vc(z.j + 1);
             if (!z.restart_pending && z.dsa)
-                IDC_TRY_CUDA(dsa_precondition(c.dims(), c.d_sigma_s, z.Vc(z.j), z.Zc(z.j), c.dsa_steps, c.d_dsa_ws, false,
-                                              c.num_sms, d_err + p, c.spin_limit, st));
+                dsa[c.dsa_steps].push_back(
+                    DsaJob{c.dims(), c.d_sigma_s, z.Vc(z.j), z.Zc(z.j), c.d_dsa_ws, d_err + p, c.spin_limit});
         }
+        for (const auto &d : dsa)
+            IDC_TRY_CUDA(dsa_precondition(d.second.data(), (int)d.second.size(), d.first, false, c0.num_sms, st));
         // lane-kernel members: out = in - P L^{-1} S in straight from the vectors; modal ones: P L^{-1} of S in, formed here
         for (size_t p = 0; p < M; ++p) {
             State &z = S[p];

@@ -17,6 +17,8 @@
 #include "device_sync.cuh"
 #include "idc_internal.hpp"
 
+#include <vector>
+
 namespace idc {
 
 namespace {
@@ -277,6 +279,237 @@ struct DsaWs {
     }
 };
 
+// ---- the same PCG in one thread-block cluster -----------------------------------------------------------------
+//
+// Grids of up to kClusterCells cells: a cluster of up to 16 blocks holds a whole problem in registers and shared
+// memory (thread l of a block owns K consecutive cells), reads its neighbours' u from the owners' shared memory, and
+// meets in the cluster barrier unit instead of at a counter in L2.  A step is bound by its two cluster barriers and the
+// latency of the reductions, not by bandwidth; the cooperative kernel's grid barriers and L2 round trips took 4.6 us a
+// step whatever the size.  Every problem of a batch is a cluster of the same launch.  Each warp's partial sums go to
+// every block and are added in one fixed order: bitwise reproducible, the same step lengths everywhere.
+constexpr int kClusterThreads = 512, kClusterWarps = kClusterThreads / 32, kMaxClusterBlocks = 16, kMaxClusterK = 8;
+constexpr int kClusterCells = kClusterThreads * kMaxClusterBlocks * kMaxClusterK;
+constexpr int kMaxJobs = 24;
+
+struct PcgJob {
+    int nx, ny, N, scale;
+    double dx, dy;
+    const double *ss, *v, *Dc, *sa, *dinv;
+    double *x;
+};
+struct PcgJobs {
+    int cg_steps;
+    PcgJob job[kMaxJobs];
+};
+static_assert(sizeof(PcgJobs) <= 4000, "kernel parameters");
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_blocks() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, unsigned rank) {   // the same place in block `rank`
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ double ld_cluster(uint32_t p) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_cluster2(uint32_t p, double a, double b) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(p), "d"(a), "d"(b) : "memory");
+}
+
+// Shared memory: u, the face coefficients to the next cell in x, the last in x and the next in y (zero at the domain's
+// edges), sigma_a with the edge terms, 1 / diagonal, [K][threads] each; the coefficient below a thread's first cell;
+// the partial sums of every warp of the cluster.
+template <int K>
+constexpr size_t cluster_smem_bytes() {
+    return sizeof(double) * ((size_t)6 * K * kClusterThreads + kClusterThreads + 2 * kMaxClusterBlocks * kClusterWarps);
+}
+
+template <int K>
+__global__ void __launch_bounds__(kClusterThreads, 1) dsa_pcg_cluster_kernel(const __grid_constant__ PcgJobs jobs) {
+    extern __shared__ __align__(16) unsigned char cluster_smem[];
+    constexpr int T = kClusterThreads, KT = K * T;
+    double *su = reinterpret_cast<double *>(cluster_smem);
+    double *cxp = su + KT, *cxm = cxp + KT, *cyp = cxm + KT, *sap = cyp + KT, *sdi = sap + KT, *cy0 = sdi + KT;
+    double *part = cy0 + T;   // [block * warps + warp][2]
+    const int rank = (int)cluster_rank(), C = (int)cluster_blocks();
+    const PcgJob &a = jobs.job[blockIdx.x / C];
+    const int nx = a.nx, ny = a.ny, n = nx * ny, l = threadIdx.x, warp = l >> 5, lane = l & 31;
+    const int first = rank * KT + l * K;   // this thread's cells: first .. first + K - 1
+    // where cell c's u is
+    auto u_addr = [&](int c) {
+        const int owner = c / KT, in = c - owner * KT;
+        return cluster_addr(su + (in % K) * T + in / K, (unsigned)owner);
+    };
+    double r[K], s[K], p[K], x[K], w[K];
+    uint32_t up[K], um[K];   // u of the next and the last cell in x
+    uint32_t ubelow = u_addr(0), uabove = ubelow;   // u below the first and above the last cell in y
+    const double ix2 = 1.0 / (a.dx * a.dx), iy2 = 1.0 / (a.dy * a.dy);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int t = first + k, at = k * T + l;
+        r[k] = s[k] = p[k] = x[k] = w[k] = 0.0;
+        up[k] = um[k] = cluster_addr(su + at, (unsigned)rank);
+        double cp = 0.0, cm = 0.0, ca = 0.0, cb = 0.0, sa = 0.0, di = 0.0;
+        if (t < n) {
+            const int i = t / ny, j = t - i * ny;
+            const double D = a.Dc[t];
+            const double ex = D / (2.0 * D + 0.25 * a.dx) / a.dx, ey = D / (2.0 * D + 0.25 * a.dy) / a.dy;
+            sa = a.sa[t];
+            di = a.dinv[t];
+            if (i > 0) cm = face_coef(D, a.Dc[t - ny]) * ix2, um[k] = u_addr(t - ny);
+            else sa += ex;
+            if (i < nx - 1) cp = face_coef(D, a.Dc[t + ny]) * ix2, up[k] = u_addr(t + ny);
+            else sa += ex;
+            if (j > 0) cb = face_coef(D, a.Dc[t - 1]) * iy2;
+            else sa += ey;
+            if (j < ny - 1) ca = face_coef(D, a.Dc[t + 1]) * iy2;
+            else sa += ey;
+            if (k == 0 && t > 0) ubelow = u_addr(t - 1);
+            if (k == K - 1 && t + 1 < n) uabove = u_addr(t + 1);
+            const size_t c = (size_t)(i + 1) * (ny + 2) + (j + 1);
+            r[k] = a.scale ? a.ss[c] * a.v[c * a.N] : a.v[c * a.N];
+        }
+        cxp[at] = cp;
+        cxm[at] = cm;
+        cyp[at] = ca;
+        sap[at] = sa;
+        sdi[at] = di;
+        if (k == 0) cy0[l] = cb;
+        su[at] = di * r[k];
+    }
+    double gamma_old = 0.0, alpha_old = 1.0;
+    for (int step = 0;; ++step) {
+        // w = C u, the partial sums of r.u and w.u
+        cluster_sync();   // every u is there
+        double g = 0.0, d = 0.0;
+        {
+            double below = ld_cluster(ubelow), cb = cy0[l], ut = su[l];
+            const double above = ld_cluster(uabove);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int at = k * T + l;
+                const double next = k + 1 < K ? su[at + T] : above, ca = cyp[at];
+                double acc = sap[at] * ut;
+                acc = fma(cxm[at], ut - ld_cluster(um[k]), acc);
+                acc = fma(cxp[at], ut - ld_cluster(up[k]), acc);
+                acc = fma(cb, ut - below, acc);
+                acc = fma(ca, ut - next, acc);
+                w[k] = acc;
+                g = fma(r[k], ut, g);
+                d = fma(acc, ut, d);
+                below = ut;
+                ut = next;
+                cb = ca;
+            }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            g += __shfl_xor_sync(kFullMask, g, off);
+            d += __shfl_xor_sync(kFullMask, d, off);
+        }
+        if (lane < C) st_cluster2(cluster_addr(part + 2 * (rank * kClusterWarps + warp), (unsigned)lane), g, d);
+        cluster_sync();   // every partial sum is there, every u has been read
+        double gamma = 0.0, delta = 0.0;
+        for (int q = lane; q < C * kClusterWarps; q += 32) {
+            const double2 v = reinterpret_cast<const double2 *>(part)[q];
+            gamma += v.x;
+            delta += v.y;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            gamma += __shfl_xor_sync(kFullMask, gamma, off);
+            delta += __shfl_xor_sync(kFullMask, delta, off);
+        }
+        const double beta = step == 0 ? 0.0 : (gamma_old != 0.0 ? gamma / gamma_old : 0.0);
+        const double den = delta - (step == 0 ? 0.0 : beta * gamma / alpha_old);
+        const double alpha = den != 0.0 ? gamma / den : 0.0;
+        gamma_old = gamma;
+        alpha_old = alpha != 0.0 ? alpha : 1.0;
+        const bool last = step + 1 >= jobs.cg_steps;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int at = k * T + l;
+            p[k] = fma(beta, p[k], su[at]);
+            s[k] = fma(beta, s[k], w[k]);
+            x[k] = fma(alpha, p[k], x[k]);
+            r[k] = fma(-alpha, s[k], r[k]);
+            su[at] = sdi[at] * r[k];
+        }
+        if (last) break;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (first + k < n) a.x[first + k] = x[k];
+}
+
+// out = v, out_00 += x (forward) or sigma_s x (transposed, ss non-null) of several problems, as dsa_correct_kernel.
+struct CorrectJob {
+    int nx, ny, N;
+    const double *v, *x, *ss;
+    double *out;
+};
+struct CorrectJobs {
+    CorrectJob job[kMaxJobs];
+};
+__global__ void dsa_correct_jobs_kernel(const __grid_constant__ CorrectJobs jobs) {
+    const CorrectJob &a = jobs.job[blockIdx.y];
+    const int cells = (a.nx + 2) * (a.ny + 2);
+    const size_t total = (size_t)cells * a.N;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+        const int c = (int)(t / a.N), k = (int)(t - (size_t)c * a.N);
+        const int i = c / (a.ny + 2), j = c - i * (a.ny + 2);
+        double val = a.v[t];
+        if (k == 0 && i >= 1 && i <= a.nx && j >= 1 && j <= a.ny) {
+            const double xc = a.x[(size_t)(i - 1) * a.ny + (j - 1)];
+            val += a.ss ? a.ss[c] * xc : xc;
+        }
+        a.out[t] = val;
+    }
+}
+
+template <int K>
+cudaError_t launch_cluster(const PcgJobs &jobs, int count, int blocks, cudaStream_t s) {
+    auto kern = dsa_pcg_cluster_kernel<K>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem_bytes<K>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(blocks * count));
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = cluster_smem_bytes<K>();
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, jobs);
+}
+
+// Blocks per cluster and cells per thread for n cells: one cell per thread while the cluster has room for them (the
+// steps are latency bound), then 2, 4, 8.
+void cluster_shape(int n, int *blocks, int *k) {
+    *k = 1;
+    while (n > kClusterThreads * kMaxClusterBlocks * *k) *k *= 2;
+    *blocks = 1;
+    while (n > kClusterThreads * *k * *blocks) *blocks *= 2;
+}
+
 }  // namespace
 
 size_t dsa_workspace_doubles(int nx, int ny) { return (size_t)nx * ny * 13 + 4 * kMaxPcgBlocks + 2; }
@@ -293,9 +526,9 @@ cudaError_t dsa_setup(const GridDims &g, const double *sigma_t, const double *si
     return e;
 }
 
-cudaError_t dsa_precondition(const GridDims &g, const double *sigma_s, const double *v, double *out, int cg_steps,
-                             double *ws, bool transpose, int num_sms, int *error, long long spin_limit,
-                             cudaStream_t s) {
+static cudaError_t dsa_precondition_grid(const GridDims &g, const double *sigma_s, const double *v, double *out,
+                                         int cg_steps, double *ws, bool transpose, int num_sms, int *error,
+                                         long long spin_limit, cudaStream_t s) {
     const int n = g.nx * g.ny;
     const DsaWs w(ws, n);
     int per_sm = 0;
@@ -333,6 +566,67 @@ cudaError_t dsa_precondition(const GridDims &g, const double *sigma_s, const dou
     dsa_correct_kernel<<<blocks_for(tot), kThreads, 0, s>>>(g.nx, g.ny, g.P * g.P, v, w.x,
                                                             transpose ? sigma_s : nullptr, out, w.count);
     return cudaGetLastError();
+}
+
+// `count` problems with one number of CG steps: those of one cluster shape share a launch; larger grids run on the
+// cooperative kernel one by one.
+cudaError_t dsa_precondition(const DsaJob *jobs, int count, int cg_steps, bool transpose, int num_sms, cudaStream_t s) {
+    auto small = [](const DsaJob &j) { return (int64_t)j.g.nx * j.g.ny <= kClusterCells; };
+    std::vector<char> done((size_t)count, 0);
+    for (int f = 0; f < count; ++f) {
+        if (done[f]) continue;
+        if (!small(jobs[f])) {
+            const DsaJob &j = jobs[f];
+            cudaError_t e = dsa_precondition_grid(j.g, j.sigma_s, j.v, j.out, cg_steps, j.ws, transpose, num_sms, j.error,
+                                                  j.spin_limit, s);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
+        int blocks = 0, k = 0, m = 0;
+        cluster_shape(jobs[f].g.nx * jobs[f].g.ny, &blocks, &k);
+        PcgJobs pj{};
+        CorrectJobs cj{};
+        size_t most = 0;
+        for (int q = f; q < count && m < kMaxJobs; ++q) {
+            const DsaJob &j = jobs[q];
+            int b = 0, kk = 0;
+            if (done[q] || !small(j)) continue;
+            cluster_shape(j.g.nx * j.g.ny, &b, &kk);
+            if (b != blocks || kk != k) continue;
+            done[q] = 1;
+            const DsaWs w(j.ws, j.g.nx * j.g.ny);
+            const int N = j.g.P * j.g.P;
+            pj.job[m] = PcgJob{j.g.nx, j.g.ny, N, transpose ? 0 : 1, j.g.dx, j.g.dy, j.sigma_s, j.v, w.Dc, w.sa, w.dinv, w.x};
+            cj.job[m] = CorrectJob{j.g.nx, j.g.ny, N, j.v, w.x, transpose ? j.sigma_s : nullptr, j.out};
+            const size_t tot = (size_t)(j.g.nx + 2) * (j.g.ny + 2) * N;
+            most = most > tot ? most : tot;
+            ++m;
+        }
+        pj.cg_steps = cg_steps;
+        cudaError_t e = k == 1   ? launch_cluster<1>(pj, m, blocks, s)
+                        : k == 2 ? launch_cluster<2>(pj, m, blocks, s)
+                        : k == 4 ? launch_cluster<4>(pj, m, blocks, s)
+                                 : launch_cluster<8>(pj, m, blocks, s);
+        if (e != cudaSuccess) {   // no such cluster on this device: one by one on the cooperative kernel
+            (void)cudaGetLastError();
+            for (int q = 0; q < count; ++q) {
+                const DsaJob &j = jobs[q];
+                int b = 0, kk = 0;
+                if (!small(j)) continue;
+                cluster_shape(j.g.nx * j.g.ny, &b, &kk);
+                if (b != blocks || kk != k) continue;
+                done[q] = 1;
+                e = dsa_precondition_grid(j.g, j.sigma_s, j.v, j.out, cg_steps, j.ws, transpose, num_sms, j.error,
+                                          j.spin_limit, s);
+                if (e != cudaSuccess) return e;
+            }
+            continue;
+        }
+        dsa_correct_jobs_kernel<<<dim3((unsigned)blocks_for(most), (unsigned)m), kThreads, 0, s>>>(cj);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace idc

@@ -289,9 +289,15 @@ cudaError_t launch_phi_combine(size_t n, const double *a, const double *b, const
 // transpose of v + E C^{-1} sigma_s R v (C symmetric).  A grid barrier that gives up sets *error.
 size_t dsa_workspace_doubles(int nx, int ny);
 cudaError_t dsa_setup(const GridDims &g, const double *sigma_t, const double *sigma_s, double *ws, cudaStream_t s);
-cudaError_t dsa_precondition(const GridDims &g, const double *sigma_s, const double *v, double *out, int cg_steps,
-                             double *ws, bool transpose, int num_sms, int *error, long long spin_limit,
-                             cudaStream_t s);
+// One application: out = v + the DSA correction of v (M v, or its transpose).
+struct DsaJob {
+    GridDims g;
+    const double *sigma_s, *v;
+    double *out, *ws;
+    int *error;             // the grid barriers' error word and bound (grids too large for a cluster)
+    long long spin_limit;
+};
+cudaError_t dsa_precondition(const DsaJob *jobs, int count, int cg_steps, bool transpose, int num_sms, cudaStream_t s);
 constexpr int kDsaLaunches = 2;
 // sum over interior cells of (a - b)^2 into *out (device double), in a fixed order; scratch holds
 // multidot_scratch_doubles() doubles

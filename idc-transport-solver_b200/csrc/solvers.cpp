@@ -118,8 +118,8 @@ Status Context::gmres(Op apply, const double *b, double *x, double abs_tol, int 
         int k = 0;   // columns built in this cycle
         for (int j = 0; j < m && its < max_its; ++j) {
             if (dsa) {
-                IDC_TRY_CUDA(dsa_precondition(dims(), d_sigma_s, Vc(j), Zc(j), dsa_steps, d_dsa_ws, dsa_mode == 2,
-                                              num_sms, d_sync + 1, spin_limit, stream));
+                const DsaJob job{dims(), d_sigma_s, Vc(j), Zc(j), d_dsa_ws, d_sync + 1, spin_limit};
+                IDC_TRY_CUDA(dsa_precondition(&job, 1, dsa_steps, dsa_mode == 2, num_sms, stream));
                 launches += kDsaLaunches;
                 if (n_extra)
                     IDC_TRY_CUDA(cudaMemcpyAsync(Zc(j) + phi_len(), Vc(j) + phi_len(), sizeof(double) * n_extra,
