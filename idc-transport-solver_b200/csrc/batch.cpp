@@ -365,6 +365,7 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
         int64_t its = 0;
         bool done = false, converged = false, restart_pending = false, records = false;
         double *in = nullptr, *out = nullptr;
+        unsigned *cgs_count = nullptr;
         double *Vc(int k) const { return V + (size_t)k * n; }
         double *Zc(int k) const { return V + (size_t)(m + 1 + k) * n; }   // flexible GMRES: Z after V_0 .. V_m
     };
@@ -398,9 +399,11 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
             IDC_TRY_CUDA(cudaMalloc(&c.d_krylov, sizeof(double) * need));
             c.krylov_len = need;
         }
-        if (!c.d_small) IDC_TRY_CUDA(cudaMalloc(&c.d_small, sizeof(double) * (128 + multidot_scratch_doubles())));
+        if (!c.d_small) IDC_TRY_CUDA(cudaMalloc(&c.d_small, sizeof(double) * (128 + cgs2_scratch_doubles())));
         if (!c.h_small) IDC_TRY_CUDA(cudaMallocHost(&c.h_small, sizeof(double) * 129));
         IDC_TRY(c.ensure_phi_buffers(7));
+        z.cgs_count = reinterpret_cast<unsigned *>(c.d_small + 128 + cgs2_scratch_doubles() - 1);
+        IDC_TRY_CUDA(cudaMemsetAsync(z.cgs_count, 0, sizeof(unsigned), st));
         z.V = c.d_krylov;
         z.b = c.phi_buf(3);
         z.x = c.phi_buf(4);
@@ -510,6 +513,7 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
             if (!z.records) IDC_TRY(scatter(z, z.in));
         }
         IDC_TRY(sweep(nullptr, nullptr, scats.data(), 1.0, tmps.data(), dt, precision, &active, true));
+        std::vector<Cgs2Job> cgs;
         for (size_t p = 0; p < M; ++p) {
             State &z = S[p];
             if (z.done) continue;
@@ -523,14 +527,15 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
                 IDC_TRY_CUDA(launch_axpby(1.0, z.b, -1.0, z.Vc(0), n, st));
                 IDC_TRY_CUDA(launch_dot(z.Vc(0), z.Vc(0), n, c.d_small + 127, c.d_small + 128, st));
             } else {                   // CGS2 against V_0 .. V_j, then |w|^2
-                const int j = z.j;
-                double *ds = c.d_small, *scratch = c.d_small + 128;
-                IDC_TRY_CUDA(launch_multidot(z.V, j + 1, n, z.Vc(j + 1), n, ds, scratch, st));
-                IDC_TRY_CUDA(launch_multiaxpy(z.Vc(j + 1), z.V, j + 1, n, ds, n, st));
-                IDC_TRY_CUDA(launch_multidot(z.V, j + 1, n, z.Vc(j + 1), n, ds + 64, scratch, st));
-                IDC_TRY_CUDA(launch_multiaxpy(z.Vc(j + 1), z.V, j + 1, n, ds + 64, n, st));
-                IDC_TRY_CUDA(launch_dot(z.Vc(j + 1), z.Vc(j + 1), n, ds + 127, scratch, st));
+                cgs.push_back(Cgs2Job{z.V, z.Vc(z.j + 1), n, z.j + 1, c.d_small + 128, c.d_small, z.cgs_count, d_err + p,
+                                      c.spin_limit});
             }
+        }
+        if (!cgs.empty()) IDC_TRY_CUDA(launch_cgs2(cgs.data(), (int)cgs.size(), c0.num_sms, st));
+        for (size_t p = 0; p < M; ++p) {
+            State &z = S[p];
+            if (z.done) continue;
+            Context &c = *z.c;
             double *ds = c.d_small;
             IDC_TRY_CUDA(cudaMemcpyAsync(c.h_small, ds, sizeof(double) * 128, cudaMemcpyDeviceToHost, st));
             IDC_TRY_CUDA(cudaMemcpyAsync(c.h_small + 128, d_err + p, sizeof(int), cudaMemcpyDeviceToHost, st));

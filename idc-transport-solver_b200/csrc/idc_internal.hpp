@@ -245,6 +245,26 @@ cudaError_t launch_reduce_phi_partials(const GridDims &g, const double *part, in
 // Krylov helpers on flat FP64 vectors of length n (device pointers; `out` arrays are device memory)
 // out[k] = V_k . w for k < nv (<= 64), in a fixed order; scratch holds multidot_scratch_doubles() doubles
 size_t multidot_scratch_doubles();
+// One CGS2 step of GMRES for several problems in one launch: w against V_0 .. V_{nv-1} (n doubles each).  coef (as the
+// solvers' d_small): [0 .. nv) and [64 .. 64 + nv) the two passes' coefficients, [127] |w|^2.  part:
+// cgs2_scratch_doubles, whose last double holds the counter: zero before the first launch (each leaves it zero).
+struct Cgs2Job {
+    const double *V;
+    double *w;
+    size_t n;
+    int nv;
+    double *part, *coef;
+    unsigned *count;
+    int *error;             // the grid barriers' error word and bound
+    long long spin_limit;
+};
+size_t cgs2_scratch_doubles();
+constexpr int kCgs2MaxJobs = 32;
+struct Cgs2Jobs {
+    int count, first[kCgs2MaxJobs + 1];
+    Cgs2Job job[kCgs2MaxJobs];
+};
+cudaError_t launch_cgs2(const Cgs2Job *jobs, int count, int num_sms, cudaStream_t s);
 cudaError_t launch_multidot(const double *V, int nv, size_t ld, const double *w, size_t n, double *out, double *scratch,
                             cudaStream_t s);
 cudaError_t launch_multiaxpy(double *w, const double *V, int nv, size_t ld, const double *c, size_t n, cudaStream_t s);

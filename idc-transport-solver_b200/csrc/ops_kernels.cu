@@ -660,6 +660,126 @@ __global__ void multiaxpy_kernel(double *__restrict__ w, const double *__restric
     }
 }
 
+// ---- one Arnoldi orthogonalisation (CGS2) ----
+// c1 = V^T w, w -= V c1, c2 = V^T w, w -= V c2, then |w|^2, in one cooperative launch for all problems of a batch: the
+// eight kernels of the separate operations (dot products in two passes, updates) cost 3-5 us each on vectors that take
+// less than a microsecond to read.  A problem has its own blocks, each thread its own elements of w (so an update and
+// the next dot product need no barrier between them), and two grid barriers; its last block to finish adds the norm.
+// Every block adds the per-block partial sums in the same order: bitwise reproducible.  The barriers are bounded.
+constexpr int kCgsThreads = 512;
+
+// Partial dot products of vectors k0 .. k0 + 3 (those below nv) with w over this block's elements.
+__device__ __forceinline__ void cgs_partials(const Cgs2Job &a, int b, int nb, double (*red)[kCgsThreads / 32]) {
+    const size_t stride = (size_t)nb * kCgsThreads;
+    for (int k0 = 0; k0 < a.nv; k0 += 4) {
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (size_t i = (size_t)b * kCgsThreads + threadIdx.x; i < a.n; i += stride) {
+            const double wi = a.w[i];
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (k0 + m < a.nv) acc[m] = fma(a.V[(size_t)(k0 + m) * a.n + i], wi, acc[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            double v = acc[m];
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if ((threadIdx.x & 31) == 0) red[m][threadIdx.x >> 5] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x < 4 && k0 + (int)threadIdx.x < a.nv) {
+            double v = red[threadIdx.x][0];
+            for (int t = 1; t < kCgsThreads / 32; ++t) v += red[threadIdx.x][t];
+            a.part[(size_t)(k0 + threadIdx.x) * nb + b] = v;
+        }
+        __syncthreads();
+    }
+}
+// The job's blocks meet for the e-th time (e = 1, 2); false if the wait gave up or another block has failed.
+__device__ __forceinline__ bool cgs_barrier(const Cgs2Job &a, unsigned e, int nb) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        __threadfence();
+        atomicAdd(a.count, 1u);
+        for (long long n = 0;; ++n) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
+            if ((int)(v - e * (unsigned)nb) >= 0) break;
+            int err = kDevOk;
+            if ((n & 63) == 63) asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(err) : "l"(a.error) : "memory");
+            if (err != kDevOk || n > a.spin_limit) {
+                atomicCAS(a.error, kDevOk, kDevTimeout);
+                ok = 0;
+                break;
+            }
+        }
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+__global__ void __launch_bounds__(kCgsThreads, 2) cgs2_kernel(const __grid_constant__ Cgs2Jobs jobs) {
+    __shared__ double red[4][kCgsThreads / 32], coef[kMaxDots];
+    __shared__ int s_last;
+    int q = 0;
+    while (q + 1 < jobs.count && (int)blockIdx.x >= jobs.first[q + 1]) ++q;
+    const Cgs2Job &a = jobs.job[q];
+    const int b = (int)blockIdx.x - jobs.first[q], nb = jobs.first[q + 1] - jobs.first[q];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t stride = (size_t)nb * kCgsThreads;
+    double norm = 0.0;
+    cgs_partials(a, b, nb, red);
+    for (int pass = 0; pass < 2; ++pass) {
+        if (!cgs_barrier(a, pass + 1, nb)) return;
+        for (int k = warp; k < a.nv; k += kCgsThreads / 32) {   // the partial sums come from L2: other blocks wrote them
+            double v = 0.0;
+            for (int t = lane; t < nb; t += 32) v += __ldcg(a.part + (size_t)pass * kMaxDots * kDotBlocks + (size_t)k * nb + t);
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if (lane == 0) {
+                coef[k] = v;
+                if (b == 0) a.coef[64 * pass + k] = v;
+            }
+        }
+        __syncthreads();
+        for (size_t i = (size_t)b * kCgsThreads + threadIdx.x; i < a.n; i += stride) {
+            double acc = a.w[i];
+            for (int k = 0; k < a.nv; ++k) acc -= coef[k] * a.V[(size_t)k * a.n + i];
+            a.w[i] = acc;
+            norm = fma(acc, acc, norm);
+        }
+        if (pass == 0) {
+            norm = 0.0;
+            Cgs2Job second = a;   // the second pass's partial sums have their own place
+            second.part = a.part + (size_t)kMaxDots * kDotBlocks;
+            cgs_partials(second, b, nb, red);
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) norm += __shfl_down_sync(0xffffffffu, norm, off);
+    __syncthreads();
+    if (lane == 0) red[0][warp] = norm;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = red[0][0];
+        for (int t = 1; t < kCgsThreads / 32; ++t) v += red[0][t];
+        a.part[b] = v;   // (the first pass's sums have been read)
+        __threadfence();
+        s_last = atomicAdd(a.count, 1u) == 3u * (unsigned)nb - 1u;
+    }
+    __syncthreads();
+    if (s_last && warp == 0) {
+        __threadfence();
+        double v = 0.0;
+        for (int t = lane; t < nb; t += 32) v += __ldcg(a.part + t);
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) {
+            a.coef[127] = v;
+            *a.count = 0u;   // armed for the next launch
+        }
+    }
+}
+
 // y = a*x + b*y
 __global__ void axpby_kernel(double a, const double *__restrict__ x, double b, double *__restrict__ y, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -747,6 +867,7 @@ __global__ void adjoint_gradient_kernel(GridDims g, const double *__restrict__ p
 }  // namespace
 
 size_t multidot_scratch_doubles() { return (size_t)kMaxDots * kDotBlocks; }
+size_t cgs2_scratch_doubles() { return 2 * (size_t)kMaxDots * kDotBlocks + 2; }   // two passes' partial sums, the counter
 
 cudaError_t launch_multidot(const double *V, int nv, size_t ld, const double *w, size_t n, double *out, double *scratch,
                             cudaStream_t s) {
@@ -756,6 +877,32 @@ cudaError_t launch_multidot(const double *V, int nv, size_t ld, const double *w,
     multidot_partial_kernel<<<dim3(bx, (nv + 3) / 4), kThreads, 0, s>>>(V, nv, ld, w, n, scratch);
     multidot_final_kernel<<<nv, 32, 0, s>>>(scratch, bx, out);
     return cudaGetLastError();
+}
+cudaError_t launch_cgs2(const Cgs2Job *jobs, int count, int num_sms, cudaStream_t s) {
+    for (int first = 0; first < count; first += kCgs2MaxJobs) {
+        Cgs2Jobs p{};
+        p.count = count - first < kCgs2MaxJobs ? count - first : kCgs2MaxJobs;
+        // every block resident: at most one per SM and problem share, by vector length
+        size_t total = 0;
+        for (int q = 0; q < p.count; ++q) {
+            if (jobs[first + q].nv < 1 || jobs[first + q].nv > kMaxDots) return cudaErrorInvalidValue;
+            total += jobs[first + q].n;
+        }
+        int at = 0;
+        for (int q = 0; q < p.count; ++q) {
+            const size_t n = jobs[first + q].n;
+            const int own = (int)((n + kCgsThreads - 1) / kCgsThreads);
+            const int share = 1 + (int)((size_t)(num_sms - 1) * n / total);   // <= num_sms + count over all problems
+            p.job[q] = jobs[first + q];
+            p.first[q] = at;
+            at += own < share ? own : share;
+        }
+        p.first[p.count] = at;
+        void *args[] = {&p};
+        cudaError_t e = cudaLaunchCooperativeKernel((const void *)cgs2_kernel, dim3(at), dim3(kCgsThreads), args, 0, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 cudaError_t launch_multiaxpy(double *w, const double *V, int nv, size_t ld, const double *c, size_t n, cudaStream_t s) {
     multiaxpy_kernel<<<blocks_for(n), kThreads, 0, s>>>(w, V, nv, ld, c, n);

@@ -76,9 +76,11 @@ Status Context::gmres(Op apply, const double *b, double *x, double abs_tol, int 
         IDC_TRY_CUDA(cudaMalloc(&d_krylov, sizeof(double) * need));
         krylov_len = need;
     }
-    if (!d_small) IDC_TRY_CUDA(cudaMalloc(&d_small, sizeof(double) * (128 + multidot_scratch_doubles())));
+    if (!d_small) IDC_TRY_CUDA(cudaMalloc(&d_small, sizeof(double) * (128 + cgs2_scratch_doubles())));
     if (!h_small) IDC_TRY_CUDA(cudaMallocHost(&h_small, sizeof(double) * 129));
     double *dot_scratch = d_small + 128;
+    unsigned *cgs_count = reinterpret_cast<unsigned *>(dot_scratch + cgs2_scratch_doubles() - 1);
+    IDC_TRY_CUDA(cudaMemsetAsync(cgs_count, 0, sizeof(unsigned), stream));   // (also after a wait that gave up)
     double *V = d_krylov;
     auto Vc = [&](int k) { return V + (size_t)k * n; };
     auto Zc = [&](int k) { return V + (size_t)(m + 1 + k) * n; };
@@ -131,12 +133,9 @@ Status Context::gmres(Op apply, const double *b, double *x, double abs_tol, int 
             // CGS2: h = V^T w, w -= V h, twice; then |w|^2.  The two coefficient columns (d_small[0..], [64..]),
             // the squared norm (d_small[127]) and the device error word reach the host in one pinned copy
             // with one synchronisation.
-            IDC_TRY_CUDA(launch_multidot(V, j + 1, n, Vc(j + 1), n, d_small, dot_scratch, stream));
-            IDC_TRY_CUDA(launch_multiaxpy(Vc(j + 1), V, j + 1, n, d_small, n, stream));
-            IDC_TRY_CUDA(launch_multidot(V, j + 1, n, Vc(j + 1), n, d_small + 64, dot_scratch, stream));
-            IDC_TRY_CUDA(launch_multiaxpy(Vc(j + 1), V, j + 1, n, d_small + 64, n, stream));
-            IDC_TRY_CUDA(launch_dot(Vc(j + 1), Vc(j + 1), n, d_small + 127, dot_scratch, stream));
-            launches += 8;
+            const Cgs2Job cgs{V, Vc(j + 1), n, j + 1, dot_scratch, d_small, cgs_count, d_sync + 1, spin_limit};
+            IDC_TRY_CUDA(launch_cgs2(&cgs, 1, num_sms, stream));
+            launches += 1;
             IDC_TRY_CUDA(cudaMemcpyAsync(h_small, d_small, sizeof(double) * 128, cudaMemcpyDeviceToHost, stream));
             IDC_TRY_CUDA(cudaMemcpyAsync(h_small + 128, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
             IDC_TRY_CUDA(cudaStreamSynchronize(stream));
