@@ -404,7 +404,11 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
     const long long dsoff = dcol * (long long)plane;              // psi doubles between them
     const long long cell0 = ((long long)xi0 - (long long)xis * rr) * (long long)cstride + j;   // step 0's column
     const long long seg0 = cell0 * (long long)plane + (long long)item.q_begin * N;             // its row segment
-    long long pf_soff = seg0 + (CHUNK ? 2 * o : (long long)(q - item.q_begin) * N);
+    const double *pf_src = a.src + (seg0 + (CHUNK ? 2 * o : (long long)(q - item.q_begin) * N));   // step t's, in order
+    const double *pf_src2 = a.src2 + (seg0 + (CHUNK ? 2 * o : (long long)(q - item.q_begin) * N));
+    auto chunk16 = [](const double *p) {   // the 16-byte boundary at or below
+        return reinterpret_cast<const double *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15);
+    };
     // parity of a row segment's address in 8-byte words at step t: par ^ (t & podd), kept running (steps s and s + D
     // share it)
     static_assert(D % 2 == 0, "steps s and s + D have the same parity");
@@ -422,7 +426,7 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
     const double *rec_src = PHI ? a.modal_src + (size_t)quadrant * RD : has_rec ? a.cell_rec : a.sigma_t;
     const long long rec_cell = PHI ? 4 * RD : has_rec ? RD : 1;   // doubles per cell
     int prow[NI], pdst[NI];
-    long long poff[NI];
+    const double *pf_rec[NI];
 #pragma unroll
     for (int h = 0; h < NI; ++h) {
         const int idx = lane + 32 * h;
@@ -431,8 +435,8 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
         pdst[h] = prow[h] * RD + (has_rec ? 2 * k : N);
         if (prow[h] >= Rw || row_w + prow[h] >= a.ny) prow[h] = -(1 << 28);   // nothing to copy: never in range
         const int r = prow[h] < 0 ? 0 : prow[h];
-        poff[h] = (((long long)xi0 - (long long)xis * r) * (long long)cstride + row_j(row_w + r)) * rec_cell +
-                  (has_rec ? 2 * k : 0);
+        pf_rec[h] = rec_src + ((((long long)xi0 - (long long)xis * r) * (long long)cstride + row_j(row_w + r)) * rec_cell +
+                               (has_rec ? 2 * k : 0));
     }
     const long long dpoff = dcol * rec_cell;
     // step t's inputs into stage slot = t % D; a cell outside the row is not copied (its results are not used)
@@ -442,33 +446,34 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
         if constexpr (CHUNK) {
             const int lim = in && has_src ? seg_n + (int)par - 2 * o : 0;
             double *d = stage + (size_t)(slot * Rw + rr) * PITCH + 2 * o;
-            const double *g = a.src + (pf_soff - (long long)par);
+            const double *g = chunk16(pf_src);
 #pragma unroll
             for (int h = 0; h < NC; ++h) cp_async16_if(d + 2 * SEG * h, g + 2 * SEG * h, lim > 2 * SEG * h);
             if constexpr (SRC2) {
                 const int lim2 = in ? seg_n + (int)par2 - 2 * o : 0;
                 double *d2 = stage2 + (size_t)(slot * Rw + rr) * PITCH + 2 * o;
-                const double *g2 = a.src2 + (pf_soff - (long long)par2);
+                const double *g2 = chunk16(pf_src2);
 #pragma unroll
                 for (int h = 0; h < NC; ++h) cp_async16_if(d2 + 2 * SEG * h, g2 + 2 * SEG * h, lim2 > 2 * SEG * h);
             }
         } else if constexpr (!PHI) {   // degree 0: a row segment's values are adjacent
-            cp_async8_if(stage + (size_t)(slot * Rw + rr) * PITCH + o, a.src + pf_soff, in && act && has_src);
+            cp_async8_if(stage + (size_t)(slot * Rw + rr) * PITCH + o, pf_src, in && act && has_src);
             if constexpr (SRC2)
-                cp_async8_if(stage2 + (size_t)(slot * Rw + rr) * PITCH + o, a.src2 + pf_soff, in && act);
+                cp_async8_if(stage2 + (size_t)(slot * Rw + rr) * PITCH + o, pf_src2, in && act);
         }
 #pragma unroll
         for (int h = 0; h < NI; ++h) {
             const bool pr = (unsigned)(t - prow[h]) < (unsigned)nx;
             double *d = recs + (size_t)slot * Rw * RD + pdst[h];
             if (has_rec)
-                cp_async16_if(d, rec_src + poff[h], pr);
+                cp_async16_if(d, pf_rec[h], pr);
             else
-                cp_async8_if(d, rec_src + poff[h], pr);
-            poff[h] += dpoff;
+                cp_async8_if(d, pf_rec[h], pr);
+            pf_rec[h] += dpoff;
         }
         cp_commit();
-        pf_soff += dsoff;
+        pf_src += dsoff;
+        if constexpr (SRC2) pf_src2 += dsoff;
     };
     // step t's raw inputs from its landed stage: the source (with the second source and the fused scattering
     // source) and sigma_t + 1/dt
@@ -544,12 +549,14 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
     double tnext[P];
 #pragma unroll
     for (int m = 0; m < P; ++m) tnext[m] = ld_ring_if(ring_in + 8u * m, reader);
-    // per-step running values of the loop: the ring slot of column s, the stage slots of steps s and s + 1, and column
-    // s - rr's cell index and psi offset
+    // per-step running values of the loop: the ring slot of column s, the stage slots of steps s and s + 1, and where
+    // column s - rr's psi and partial moments go
     uint32_t ring_slot = ring_in;
     int sl = 0, sl1 = 1;
-    long long fin_cidx = cell0;
-    long long fin_ooff = seg0;
+    double *out_p = a.out + seg0;   // column s - rr's row segment
+    const int mk = SEG >= 16 ? (o < N ? o : N - 1) : 0;   // 16-wide segments: the moment this lane sums
+    double *phi_p = phi_base + cell0 * N + mk;
+    const long long dphi = dcol * N;
     TC gprev[P];
 #pragma unroll
     for (int m = 0; m < P; ++m) gprev[m] = TC(0);
@@ -570,7 +577,7 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
             const bool p = reader && s < nx;
             bool wait = cout >= credit && cout < nx;
 #pragma unroll
-            for (int m = 0; m < P; ++m) wait |= p && is_sentinel(tnext[m]);
+            for (int m = 0; m < P; ++m) wait |= p && __double2hiint(tnext[m]) == (int)(kTraceSentinel >> 32);   // (no quiet NaN has it)
             if (__builtin_expect(__any_sync(kFullMask, wait), 0)) {
                 const StepWait<P> w = wait_for_step<P>(ring_slot, p, consumed + 4u, cout, credit, nx, a.error,
                                                        a.spin_limit, lane);
@@ -631,7 +638,7 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
             if constexpr (OBUF) {   // the 16-byte chunks of the row segment
                 const int body = (seg_n - (int)opar) & ~1;
                 const int lim = pb ? body - 2 * o : 0;
-                double *dst = a.out + fin_ooff;
+                double *dst = out_p;
                 const double2 *ov = reinterpret_cast<const double2 *>(obuf + 2 * opar + 2 * o);
 #pragma unroll
                 for (int h = 0; h < NC; ++h) st_f64x2_if(dst + opar + 2 * o + 2 * SEG * h, ov[SEG * h], lim > 2 * SEG * h);
@@ -640,7 +647,7 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
                     st_f64_if(dst + seg_n - 1, double(x[N - 1]), pb && o + 1 == item.q_count && (int)opar + body != seg_n);
                 }
             } else if constexpr (!PHI) {
-                double *dst = a.out + fin_ooff + o * N;
+                double *dst = out_p + o * N;
                 if constexpr (N == 4) {   // a lane's block is 32 bytes
                     if (out_align == 0) {
                         st_f64x4_if(dst, double(x[0]), double(x[1]), double(x[2]), double(x[3]), pb && act);
@@ -659,10 +666,8 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
             // sum's 15 dependent adds cost 4% of the 256x256 Q2 S16 sweep on B200); narrower ones by a shuffle
             // butterfly (measured on B200: each is the faster one at its width).
             const bool pp = inrow && phi_base != nullptr;
-            double *pt = phi_base + fin_cidx * N;
             if constexpr (SEG >= 16) {
-                const int k = o < N ? o : N - 1;
-                const double2 *mv = reinterpret_cast<const double2 *>(mbuf + k * kMomStride + rr * SEG);
+                const double2 *mv = reinterpret_cast<const double2 *>(mbuf + mk * kMomStride + rr * SEG);
                 double part[SEG / 2];   // a pairwise tree in ordinate order: 4 dependent adds, not 15
 #pragma unroll
                 for (int h = 0; h < SEG / 2; ++h) {
@@ -673,14 +678,14 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
                 for (int w = SEG / 4; w >= 1; w /= 2)
 #pragma unroll
                     for (int h = 0; h < w; ++h) part[h] = part[2 * h] + part[2 * h + 1];
-                st_f64_if(pt + k, part[0], pp && o < N);
+                st_f64_if(phi_p, part[0], pp && o < N);
             } else {
 #pragma unroll
                 for (int k = 0; k < N; ++k) x[k] = wv * x[k];
                 int lo = 0, hi = N;
                 segment_sums<N, SEG>(x, o, &lo, &hi);
 #pragma unroll
-                for (int i = 0; i < (N + SEG - 1) / SEG; ++i) st_f64_if(pt + lo + i, double(x[i]), pp && lo + i < hi);
+                for (int i = 0; i < (N + SEG - 1) / SEG; ++i) st_f64_if(phi_p + lo + i, double(x[i]), pp && lo + i < hi);
             }
         }
         // ---- the copies of step s + D, into the stage of step s (read in the last iteration); step s + 2's inputs ----
@@ -697,8 +702,8 @@ __device__ __forceinline__ void run_rows(const SweepArgs &a, const SweepItem &it
 #pragma unroll
         for (int m = 0; m < P; ++m) tnext[m] = ld_ring_if(ring_slot + 8u * m, reader && s + 1 < nx);
         opar ^= podd;
-        fin_cidx += dcol;
-        fin_ooff += dsoff;
+        phi_p += dphi;
+        out_p += dsoff;
     }
     cp_wait<0>();
 }
