@@ -379,7 +379,7 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
     std::vector<State> S(M);
     auto scatter = [&](State &z, const double *phi) -> Status {
         if (z.records)
-            IDC_TRY_CUDA(launch_cell_records(z.c->dims(), z.c->d_sigma_t, z.c->d_sigma_s, phi, z.scat, st));
+            IDC_TRY_CUDA(launch_cell_records(z.c->dims(), z.c->d_sigma_t, z.c->d_sigma_s, phi, z.scat, nullptr, st));
         else
             IDC_TRY_CUDA(launch_scatter_moments(z.c->dims(), z.c->d_sigma_s, phi, z.scat, st));
         return Status::ok();
@@ -527,14 +527,17 @@ Status Batch::gmres_solve(double *const *psi_inout, double dt, double abs_tol, i
                 IDC_TRY_CUDA(launch_axpby(1.0, z.b, -1.0, z.Vc(0), n, st));
                 IDC_TRY_CUDA(launch_dot(z.Vc(0), z.Vc(0), n, c.d_small + 127, c.d_small + 128, st));
             } else {                   // CGS2 against V_0 .. V_j, then |w|^2
-                cgs.push_back(Cgs2Job{z.V, z.Vc(z.j + 1), n, z.j + 1, c.d_small + 128, c.d_small, z.cgs_count, d_err + p,
-                                      c.spin_limit});
+                cgs.push_back(Cgs2Job{z.V, z.Vc(z.j + 1), n, z.j + 1, c.d_small + 128, c.d_small, c.h_small, z.cgs_count,
+                                      d_err + p, c.spin_limit});
+                const int unwritten = -1;   // a launch that gives up leaves the error word here unwritten
+                std::memcpy(c.h_small + 128, &unwritten, sizeof(int));
             }
         }
         if (!cgs.empty()) IDC_TRY_CUDA(launch_cgs2(cgs.data(), (int)cgs.size(), c0.num_sms, st));
         for (size_t p = 0; p < M; ++p) {
             State &z = S[p];
             if (z.done) continue;
+            if (!z.restart_pending) continue;   // the CGS2 launch writes its results to the host
             Context &c = *z.c;
             double *ds = c.d_small;
             IDC_TRY_CUDA(cudaMemcpyAsync(c.h_small, ds, sizeof(double) * 128, cudaMemcpyDeviceToHost, st));

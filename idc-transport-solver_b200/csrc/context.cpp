@@ -51,6 +51,7 @@ Context::~Context() {
     cudaFree(d_reflect_g_);
     cudaFree(d_reflect_vec_);
     cudaFree(d_scalar_);
+    cudaFreeHost(h_pin_);
     cudaFree(d_xi);
     cudaFree(d_eta);
     cudaFree(d_w);
@@ -103,6 +104,7 @@ Status Context::init() {
     IDC_TRY_CUDA(cudaEventCreate(&ev0));
     IDC_TRY_CUDA(cudaEventCreate(&ev1));
     IDC_TRY_CUDA(cudaMalloc(&d_scalar_, sizeof(double) * (4 + multidot_scratch_doubles())));   // + dot scratch
+    IDC_TRY_CUDA(cudaMallocHost(&h_pin_, sizeof(double) * 2));
     // IDC_SWEEP_KERNEL=modal|warp|rowsync selects another sweep kernel than the lane-pipelined one
     if (const char *k = std::getenv("IDC_SWEEP_KERNEL")) {
         const std::string v(k);
@@ -383,8 +385,7 @@ Status Context::source_iteration_periodic(const double *src, double *psi_out, do
         launches += it > 1 ? 2 : 1;
         IDC_TRY(smv(1.0, 1.0, phi_last, psi_out));
         IDC_TRY(sweep(psi_out, psi_out, dt, phi_cur, precision));
-        IDC_TRY(l2dist(phi_cur, phi_last, &e));
-        IDC_TRY(check_device_error());
+        IDC_TRY(l2dist(phi_cur, phi_last, &e, true));
     }
     if (iters) *iters = it;
     if (err) *err = e;
@@ -424,8 +425,7 @@ Status Context::source_iteration_reflecting(const double *src, double *psi_out, 
         IDC_TRY_CUDA(launch_smv(dims(), 1.0, 1.0, d_sigma_s, phi_last, psi_out, stream));
         launches += 1;
         IDC_TRY(reflect_quadrants(psi_out, dt, phi_cur, precision));
-        IDC_TRY(l2dist(phi_cur, phi_last, &e));
-        IDC_TRY(check_device_error());
+        IDC_TRY(l2dist(phi_cur, phi_last, &e, true));
     }
     if (iters) *iters = it;
     if (err) *err = e;
@@ -487,6 +487,8 @@ Status Context::set_sigma(const double *sigma_t, const double *sigma_s, int loc)
         IDC_TRY_CUDA(cudaMemcpy(d_sigma_s, sigma_s, sizeof(double) * sig_len(), kind));
     else
         IDC_TRY_CUDA(cudaMemset(d_sigma_s, 0, sizeof(double) * sig_len()));
+    // (the copies above may still be under way when they return, and the context's stream does not wait for theirs)
+    IDC_TRY_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     have_sigma = true;
     return Status::ok();
 }
@@ -847,9 +849,14 @@ Status Context::sweep_host_many(int64_t count, const double *const *srcs, double
 }
 
 Status Context::check_device_error() {
-    int err = 0;
-    IDC_TRY_CUDA(cudaMemcpyAsync(&err, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_ + 1, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
+    return report_device_error();
+}
+
+Status Context::report_device_error() {
+    int err = 0;
+    std::memcpy(&err, h_pin_ + 1, sizeof(int));
     if (err != kDevOk) {
         IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 1, 0, sizeof(int), stream));
         if (d_trace)
@@ -979,13 +986,19 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
     const bool phi_only = active == kLane && !src && !out && phi && !src2 && a.phi_part && moments_fast_path;
 
     // queue head and progress flags start at zero; the error word is kept until checked
-    IDC_TRY_CUDA(cudaMemsetAsync(d_sync, 0, sizeof(int), stream));
+    // (the queue head by the first helper kernel that runs, else by a memset)
+    int *reset = d_sync;
     if (active == kRowSync)   // the only kernel with progress flags
         IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 2, 0, sizeof(int) * n_items, stream));
     if (a.phi) IDC_TRY_CUDA(cudaMemsetAsync(phi, 0, sizeof(double) * phi_len(), stream));
-    if (active != kModal && active != kLane && !capturing) IDC_TRY_CUDA(cudaEventRecord(ev0, stream));
+    if (active != kModal && active != kLane) {
+        IDC_TRY_CUDA(cudaMemsetAsync(reset, 0, sizeof(int), stream));
+        if (!capturing) IDC_TRY_CUDA(cudaEventRecord(ev0, stream));
+    }
     if (active == kModal || active == kLane) {
-        if (src && !adjoint) {   // inflow traces of the ghost cells (packed modal, or physical for the refined mode)
+        if (src && !adjoint && keep_inflow_ && inflow_len > 0) {   // (the same source's, from the last sweep)
+            a.inflow = d_inflow;
+        } else if (src && !adjoint) {   // inflow traces of the ghost cells (packed modal, or physical for the refined mode)
             const size_t need = (size_t)(nx + ny) * nq * P;
             if (inflow_len < need) {
                 cudaFree(d_inflow);
@@ -995,7 +1008,8 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
                 inflow_len = need;
             }
             IDC_TRY_CUDA(launch_inflow_traces(P, precision != IDC_PREC_FP32_REFINED, src, d_xi, d_eta, (int)nx,
-                                              (int)ny, (int)nq, d_inflow, stream));
+                                              (int)ny, (int)nq, d_inflow, reset, stream));
+            reset = nullptr;
             launches += 1;
             a.inflow = d_inflow;
         }
@@ -1010,7 +1024,8 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
                 msrc_len = need;
             }
             IDC_TRY_CUDA(launch_modal_sources(dims(), d_sigma_t, adjoint ? nullptr : d_sigma_s, phi_scatter,
-                                              adjoint ? 1.0 : scatter_scale, adjoint, d_msrc, stream));
+                                              adjoint ? 1.0 : scatter_scale, adjoint, d_msrc, reset, stream));
+            reset = nullptr;
             launches += 1;
             a.modal_src = d_msrc;
             a.phi_scatter = nullptr;
@@ -1028,7 +1043,8 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
             }
             if (active == kLane) {
                 IDC_TRY_CUDA(launch_cell_records(dims(), d_sigma_t, adjoint ? nullptr : d_sigma_s, phi_scatter, d_scat,
-                                                 stream));
+                                                 reset, stream));
+                reset = nullptr;
                 a.cell_rec = d_scat;
                 a.phi_scatter = nullptr;
             } else {
@@ -1038,6 +1054,7 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
             launches += 1;
             a.sigma_s = nullptr;
         }
+        if (reset) IDC_TRY_CUDA(cudaMemsetAsync(reset, 0, sizeof(int), stream));
         if (!capturing) IDC_TRY_CUDA(cudaEventRecord(ev0, stream));   // the timing covers the sweep kernel alone
         if (active == kLane)
             IDC_TRY_CUDA(launch_sweep_lane(P, precision, a, grid, stream));
@@ -1050,7 +1067,8 @@ Status Context::sweep(const double *src, double *out, double dt, double *phi, in
     if (!capturing) IDC_TRY_CUDA(cudaEventRecord(ev1, stream));
     launches += 1;
     if (a.phi_part && phi_only) {
-        IDC_TRY_CUDA(launch_reduce_modal_partials(dims(), d_phi_part, quad_slots, phi_len(), adjoint, minuend, phi, stream));
+        IDC_TRY_CUDA(launch_reduce_modal_partials(dims(), d_phi_part, quad_slots, phi_len(), adjoint, minuend,
+                                                  adjoint && minuend ? d_sigma_s : nullptr, phi, stream));
         launches += 1;
     } else if (a.phi_part && !skip_reduce_) {
         IDC_TRY_CUDA(launch_reduce_phi_partials(dims(), d_phi_part, items_per_rb, phi_len(), phi, stream));
@@ -1137,14 +1155,14 @@ Status Context::transport_residual_transpose(const double *z, double *y, double 
     return Status::ok();
 }
 
-Status Context::l2dist(const double *a, const double *b, double *out_host) {
+Status Context::l2dist(const double *a, const double *b, double *out_host, bool checked) {
     IDC_TRY_CUDA(launch_l2dist2(dims(), a, b, d_scalar_, d_scalar_ + 4, stream));
     launches += 2;
-    double v = 0;
-    IDC_TRY_CUDA(cudaMemcpyAsync(&v, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
+    IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
+    if (checked) IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_ + 1, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
-    *out_host = std::sqrt(v);
-    return Status::ok();
+    *out_host = std::sqrt(h_pin_[0]);
+    return checked ? report_device_error() : Status::ok();
 }
 
 // SISolver::Solve, linear_solvers/Abstract/ImplicitSolver/SISolver.cpp:190-254.  The copy of the
@@ -1160,12 +1178,16 @@ Status Context::source_iteration(const double *src, double *psi_out, double dt, 
     IDC_TRY_CUDA(cudaMemsetAsync(phi_last, 0, sizeof(double) * phi_len(), stream));
     int64_t it = 0;
     double e = INFINITY;
+    struct KeepInflow {   // the source does not change between the iterations: its inflow traces are formed by the first
+        bool &on;
+        ~KeepInflow() { on = false; }
+    } keep{keep_inflow_};
     while (it < max_its && e > abs_tol) {
         ++it;
         std::swap(phi_cur, phi_last);
         IDC_TRY(sweep(src, psi_out, dt, phi_cur, precision, phi_last, 1.0));
-        IDC_TRY(l2dist(phi_cur, phi_last, &e));
-        IDC_TRY(check_device_error());
+        keep_inflow_ = true;
+        IDC_TRY(l2dist(phi_cur, phi_last, &e, true));
     }
     // Like the reference, reaching max_its is not an error: the caller reads *err.
     if (iters) *iters = it;

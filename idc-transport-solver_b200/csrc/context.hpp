@@ -55,7 +55,9 @@ public:
     Status smv(double alpha, double beta, const double *phi, double *psi);
     Status lmv(double alpha, double beta, const double *x, double *y);
     Status transport_residual(const double *psi, const double *phi, double *res);   // (L - S P) psi, phi = P psi
-    Status l2dist(const double *a, const double *b, double *out_host);
+    // |a - b|; checked: and the device error word with it, as check_device_error, in one synchronisation
+    Status l2dist(const double *a, const double *b, double *out_host, bool checked = false);
+    Status report_device_error();   // a recorded error: clears it, re-arms the trace buffers, IDC_ERR_TIMEOUT
     Status source_iteration(const double *src, double *psi_out, double dt, double abs_tol, int64_t max_its,
                             int precision, int64_t *iters, double *err);
     // phi_guess (optional, moment-sized, device): GMRES starts from it instead of zero (reflecting or periodic
@@ -167,6 +169,7 @@ public:
     double *d_trace = nullptr;     // warp / modal kernel: per-item last-row traces (sentinel-armed)
     double *d_inflow = nullptr;    // modal kernel: inflow traces of the ghost cells
     size_t inflow_len = 0;
+    bool keep_inflow_ = false;     // source iteration: d_inflow holds this source's traces
     double *d_scat = nullptr;      // lane kernel: cell records; modal kernel: the moments sigma_s phi / (4 pi)
     size_t scat_len = 0;
     double *d_src2mix = nullptr;   // src + scale src2 when the second source's stages do not fit
@@ -270,6 +273,7 @@ private:
     double *d_ones_ = nullptr;              // nq ones: unweighted moment sums through the Pmv kernel
     std::vector<double *> idc_psi_, idc_phi_;
     double *d_scalar_ = nullptr;
+    double *h_pin_ = nullptr;               // pinned: a reduction's result, the device error word (small reads)
 };
 
 }  // namespace idc

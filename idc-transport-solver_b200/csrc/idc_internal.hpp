@@ -152,9 +152,10 @@ int sweep_modal_threads(int P, int wn);
 int sweep_modal_fit_wn(int P, int precision, int wn, int G, int seg);
 // Inflow traces of the ghost cells of `src` for the modal kernel: out[(k * nq + q) * P + m], k < nx the
 // ghost row below column k, k >= nx the ghost column left of row k - nx (sweep order); packed modal
-// coefficients if `modal`, else sign-flipped physical traces.
+// coefficients if `modal`, else sign-flipped physical traces.  reset (nullable; also of the other kernels that run before
+// a sweep): an int set to zero, the sweep's queue head.
 cudaError_t launch_inflow_traces(int P, bool modal, const double *src, const double *xi, const double *eta, int nx,
-                                 int ny, int nq, double *out, cudaStream_t stream);
+                                 int ny, int nq, double *out, int *reset, cudaStream_t stream);
 // Bit pattern of an unwritten trace slot: a signalling-NaN payload that floating-point arithmetic never
 // produces (arithmetic returns quiet NaNs).
 constexpr unsigned long long kTraceSentinel = 0x7FF4DEADBEEFCAFEull;
@@ -172,14 +173,15 @@ struct GridDims {
 // sweep sums w_q Z (Z for the transposed sweep) in the packed basis per ordinate chunk, and the reduction transforms
 // each quadrant's sum back once per cell: phi = sum_k flip_k(V (sum_{slots of k} part) V^T), slots
 // [slot_begin[k], slot_begin[k+1]) of quadrant k, interior cells in a fixed order, ghost cells zero; with
-// `minuend` x the output is x - phi (the Peierls operator's).
+// `minuend` x the output is x - phi (the Peierls operator's), with sigma_s too x - sigma_s phi / (4 pi) (its transpose's).
 cudaError_t launch_modal_sources(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
-                                 double scale, bool adjoint, double *out, cudaStream_t s);
+                                 double scale, bool adjoint, double *out, int *reset, cudaStream_t s);
 cudaError_t launch_reduce_modal_partials(const GridDims &g, const double *part, const int slot_begin[5], size_t stride,
-                                         bool adjoint, const double *minuend, double *phi, cudaStream_t s);
+                                         bool adjoint, const double *minuend, const double *sigma_s, double *phi,
+                                         cudaStream_t s);
 // The records of SweepArgs::cell_rec: sigma_s phi / (4 pi) (phi itself with sigma_s null), then sigma_t.
 cudaError_t launch_cell_records(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
-                                double *out, cudaStream_t s);
+                                double *out, int *reset, cudaStream_t s);
 cudaError_t launch_pmv(const GridDims &g, double alpha, double beta, const double *w, const double *psi,
                        double *phi, cudaStream_t s);
 cudaError_t launch_smv(const GridDims &g, double alpha, double beta, const double *sigma_s, const double *phi,
@@ -246,14 +248,15 @@ cudaError_t launch_reduce_phi_partials(const GridDims &g, const double *part, in
 // out[k] = V_k . w for k < nv (<= 64), in a fixed order; scratch holds multidot_scratch_doubles() doubles
 size_t multidot_scratch_doubles();
 // One CGS2 step of GMRES for several problems in one launch: w against V_0 .. V_{nv-1} (n doubles each).  coef (as the
-// solvers' d_small): [0 .. nv) and [64 .. 64 + nv) the two passes' coefficients, [127] |w|^2.  part:
+// solvers' d_small): [0 .. nv) and [64 .. 64 + nv) the two passes' coefficients, [127] |w|^2; host
+// (pinned): the same, and the error word in the int at [128].  part:
 // cgs2_scratch_doubles, whose last double holds the counter: zero before the first launch (each leaves it zero).
 struct Cgs2Job {
     const double *V;
     double *w;
     size_t n;
     int nv;
-    double *part, *coef;
+    double *part, *coef, *host;
     unsigned *count;
     int *error;             // the grid barriers' error word and bound
     long long spin_limit;

@@ -773,9 +773,16 @@ __global__ void __launch_bounds__(kCgsThreads, 2) cgs2_kernel(const __grid_const
         double v = 0.0;
         for (int t = lane; t < nb; t += 32) v += __ldcg(a.part + t);
         for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        for (int k = lane; k < a.nv; k += 32) {
+            a.host[k] = __ldcg(a.coef + k);
+            a.host[64 + k] = __ldcg(a.coef + 64 + k);
+        }
         if (lane == 0) {
-            a.coef[127] = v;
+            a.host[127] = v;
             *a.count = 0u;   // armed for the next launch
+            int err;
+            asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(err) : "l"(a.error) : "memory");
+            *reinterpret_cast<int *>(a.host + 128) = err;
         }
     }
 }

@@ -36,8 +36,9 @@ Status bad(int code, const std::string &m) {
 Status Context::dot_host(const double *x, const double *y, size_t n, double *out) {
     IDC_TRY_CUDA(launch_dot(x, y, n, d_scalar_, d_scalar_ + 4, stream));
     launches += 2;
-    IDC_TRY_CUDA(cudaMemcpyAsync(out, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
+    IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
+    *out = h_pin_[0];
     return Status::ok();
 }
 
@@ -131,17 +132,20 @@ Status Context::gmres(Op apply, const double *b, double *x, double abs_tol, int 
                 IDC_TRY(apply(Vc(j), Vc(j + 1)));
             }
             // CGS2: h = V^T w, w -= V h, twice; then |w|^2.  The two coefficient columns (d_small[0..], [64..]),
-            // the squared norm (d_small[127]) and the device error word reach the host in one pinned copy
-            // with one synchronisation.
-            const Cgs2Job cgs{V, Vc(j + 1), n, j + 1, dot_scratch, d_small, cgs_count, d_sync + 1, spin_limit};
+            // the squared norm ([127]) and the device error word ([128]) are written to pinned host memory by the launch.
+            const Cgs2Job cgs{V, Vc(j + 1), n, j + 1, dot_scratch, d_small, h_small, cgs_count, d_sync + 1, spin_limit};
+            // a launch that gives up leaves the error word here unwritten
+            const int unwritten = -1;
+            std::memcpy(h_small + 128, &unwritten, sizeof(int));
             IDC_TRY_CUDA(launch_cgs2(&cgs, 1, num_sms, stream));
             launches += 1;
-            IDC_TRY_CUDA(cudaMemcpyAsync(h_small, d_small, sizeof(double) * 128, cudaMemcpyDeviceToHost, stream));
-            IDC_TRY_CUDA(cudaMemcpyAsync(h_small + 128, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
             IDC_TRY_CUDA(cudaStreamSynchronize(stream));
             int dev_err = 0;
             std::memcpy(&dev_err, h_small + 128, sizeof(int));
-            if (dev_err != kDevOk) IDC_TRY(check_device_error());   // re-arms the sweep state, returns the error
+            if (dev_err != kDevOk) {
+                IDC_TRY(check_device_error());   // re-arms the sweep state, returns the error
+                return bad(IDC_ERR_TIMEOUT, "a device-side wait gave up (bounded spin) in the orthogonalisation");
+            }
             double hn = std::sqrt(h_small[127]);
             for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = h_small[i] + h_small[64 + i];
             H[(size_t)(j + 1) * m + j] = hn;
@@ -265,10 +269,13 @@ Status Context::gmres_peierls_boundary(const double *src, double *psi_out, doubl
     auto op = [&](const double *in, double *out) { return apply_peierls_boundary(in, out, tmp, dt, precision); };
     IDC_TRY(gmres(op, b, x, abs_tol, restart, max_its, iters_out, &resid, &converged, precond_kind == 1 ? 1 : 0,
                   ng));
-    IDC_TRY_CUDA(cudaMemcpyAsync(psi_out, src, sizeof(double) * psi_len(), cudaMemcpyDeviceToDevice, stream));
-    IDC_TRY(reflect_ghosts(psi_out, x + np, false));
-    IDC_TRY(smv(1.0, 1.0, x, psi_out));
-    IDC_TRY(boundary_sweep(psi_out, dt, nullptr, precision));
+    if (src != psi_out)
+        IDC_TRY_CUDA(cudaMemcpyAsync(psi_out, src, sizeof(double) * psi_len(), cudaMemcpyDeviceToDevice, stream));
+    if (converged || src != psi_out) {   // in place the source outlives a solve that failed
+        IDC_TRY(reflect_ghosts(psi_out, x + np, false));
+        IDC_TRY(smv(1.0, 1.0, x, psi_out));
+        IDC_TRY(boundary_sweep(psi_out, dt, nullptr, precision));
+    }
     IDC_TRY(check_device_error());
     if (resid_out) *resid_out = resid;
     if (!converged)
@@ -297,8 +304,8 @@ Status Context::gmres_peierls(const double *src, double *psi_out, double dt, dou
         IDC_TRY_CUDA(cudaMemcpyAsync(x, phi_guess, sizeof(double) * phi_len(), cudaMemcpyDeviceToDevice, stream));
     IDC_TRY(gmres(op, b, x, abs_tol, restart, max_its, iters_out, &resid, &converged, precond_kind == 1 ? 1 : 0, 0,
                   phi_guess != nullptr));
-    // psi = L^{-1} (S phi + Q)  (PETScPeierlsSolver.cpp:504-505)
-    IDC_TRY(sweep(src, psi_out, dt, nullptr, precision, x, 1.0));
+    // psi = L^{-1} (S phi + Q)  (PETScPeierlsSolver.cpp:504-505); in place the source outlives a solve that failed
+    if (converged || src != psi_out) IDC_TRY(sweep(src, psi_out, dt, nullptr, precision, x, 1.0));
     IDC_TRY(check_device_error());
     if (resid_out) *resid_out = resid;
     if (!converged)
@@ -350,7 +357,7 @@ Status Context::gmres_peierls_ir(const double *src, double *psi_out, double dt, 
         IDC_TRY_CUDA(launch_axpby(-1.0, ax, 1.0, r, n, stream));
         launches += 3;
     }
-    IDC_TRY(sweep(src, psi_out, dt, nullptr, IDC_PREC_FP64, x, 1.0));
+    if (converged || src != psi_out) IDC_TRY(sweep(src, psi_out, dt, nullptr, IDC_PREC_FP64, x, 1.0));
     IDC_TRY(check_device_error());
     if (iters_out) *iters_out = total;
     if (resid_out) *resid_out = resid;
@@ -373,6 +380,8 @@ Status Context::set_preconditioner(int kind, int inner_steps) {
 Status Context::apply_peierls_adjoint(const double *x, double *y, double *tmp_phi, double dt, int precision) {
     if (periodic_ || reflect_mask)
         return bad(IDC_ERR_UNSUPPORTED, "adjoint solves with periodic or reflecting edges");
+    if (kernel_for(precision) == kLane && moments_fast_path && !allreduce_fn)   // in the reduction
+        return sweep(nullptr, nullptr, dt, y, precision, x, 1.0, true, nullptr, 0.0, x);
     IDC_TRY(sweep(nullptr, nullptr, dt, tmp_phi, precision, x, 1.0, true));
     IDC_TRY_CUDA(launch_adjoint_scatter(dims(), d_sigma_s, x, tmp_phi, y, stream));
     launches += 1;

@@ -75,7 +75,8 @@ __device__ __forceinline__ void modal_sources(int nx, int ny, const double *__re
 
 template <int P, bool ADJ>
 __global__ void modal_sources_kernel(GridDims g, const double *__restrict__ sigma_t, const double *__restrict__ sigma_s,
-                                     const double *__restrict__ phi, double scale, double *__restrict__ out) {
+                                     const double *__restrict__ phi, double scale, double *__restrict__ out, int *reset) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && reset) *reset = 0;
     modal_sources<P, ADJ>(g.nx, g.ny, sigma_t, sigma_s, phi, scale, out);
 }
 // every problem of a batch's table (grid.y) that is not left out
@@ -90,7 +91,8 @@ __global__ void modal_sources_batched_kernel(const SweepArgs *__restrict__ table
 // The records of every interior cell: sigma_s phi / (4 pi) (or phi itself without sigma_s), sigma_t.
 template <int P>
 __global__ void cell_records_kernel(GridDims g, const double *__restrict__ sigma_t, const double *__restrict__ sigma_s,
-                                    const double *__restrict__ phi, double *__restrict__ out) {
+                                    const double *__restrict__ phi, double *__restrict__ out, int *reset) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && reset) *reset = 0;
     constexpr int N = P * P, RD = cell_record_doubles(P);
     const size_t total = (size_t)g.nx * g.ny * RD;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -117,7 +119,7 @@ struct SlotBounds {
 template <int P, bool ADJ>
 __device__ __forceinline__ void reduce_modal_partials(int nx, int ny, const double *__restrict__ part, const SlotBounds &sb,
                                                       size_t stride, const double *__restrict__ minuend,
-                                                      double *__restrict__ phi) {
+                                                      const double *__restrict__ sigma_s, double *__restrict__ phi) {
     constexpr int N = P * P;
     const size_t total = (size_t)(nx + 2) * (ny + 2);
     for (size_t cidx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; cidx < total;
@@ -126,7 +128,8 @@ __device__ __forceinline__ void reduce_modal_partials(int nx, int ny, const doub
         double acc[N];
 #pragma unroll
         for (int m = 0; m < N; ++m) acc[m] = 0.0;
-        if (i >= 1 && i <= nx && j >= 1 && j <= ny) {
+        const bool interior = i >= 1 && i <= nx && j >= 1 && j <= ny;
+        if (interior) {
             for (int k = 0; k < 4; ++k) {
                 if (sb.b[k + 1] == sb.b[k]) continue;
                 double M[N], x[N];
@@ -145,13 +148,17 @@ __device__ __forceinline__ void reduce_modal_partials(int nx, int ny, const doub
             }
         }
 #pragma unroll
-        for (int m = 0; m < N; ++m) phi[cidx * N + m] = minuend ? minuend[cidx * N + m] - acc[m] : acc[m];
+        for (int m = 0; m < N; ++m) {
+            const double v = sigma_s && interior ? sigma_s[cidx] / (4.0 * M_PI) * acc[m] : acc[m];
+            phi[cidx * N + m] = minuend ? minuend[cidx * N + m] - v : v;
+        }
     }
 }
 template <int P, bool ADJ>
 __global__ void reduce_modal_partials_kernel(GridDims g, const double *__restrict__ part, SlotBounds sb, size_t stride,
-                                             const double *__restrict__ minuend, double *__restrict__ phi) {
-    reduce_modal_partials<P, ADJ>(g.nx, g.ny, part, sb, stride, minuend, phi);
+                                             const double *__restrict__ minuend, const double *__restrict__ sigma_s,
+                                             double *__restrict__ phi) {
+    reduce_modal_partials<P, ADJ>(g.nx, g.ny, part, sb, stride, minuend, sigma_s, phi);
 }
 template <int P>
 __global__ void reduce_modal_batched_kernel(const SweepArgs *__restrict__ table) {
@@ -159,7 +166,7 @@ __global__ void reduce_modal_batched_kernel(const SweepArgs *__restrict__ table)
     if (a.skip) return;
     SlotBounds sb;
     for (int k = 0; k < 5; ++k) sb.b[k] = a.slot_begin[k];
-    reduce_modal_partials<P, false>(a.nx, a.ny, a.phi_part, sb, a.phi_slot_stride, a.phi_scatter, a.phi);
+    reduce_modal_partials<P, false>(a.nx, a.ny, a.phi_part, sb, a.phi_slot_stride, a.phi_scatter, nullptr, a.phi);
 }
 
 int blocks_for(size_t n) {
@@ -216,44 +223,45 @@ cudaError_t launch_sweep_lane(int P, int precision, const SweepArgs &args, int g
 }
 
 cudaError_t launch_modal_sources(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
-                                 double scale, bool adjoint, double *out, cudaStream_t s) {
+                                 double scale, bool adjoint, double *out, int *reset, cudaStream_t s) {
     const int b = blocks_for((size_t)g.nx * g.ny * 4);
     switch (g.P + (adjoint ? 4 : 0)) {
-        case 1: modal_sources_kernel<1, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
-        case 2: modal_sources_kernel<2, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
-        case 3: modal_sources_kernel<3, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
-        case 5: modal_sources_kernel<1, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
-        case 6: modal_sources_kernel<2, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
-        case 7: modal_sources_kernel<3, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out); break;
+        case 1: modal_sources_kernel<1, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
+        case 2: modal_sources_kernel<2, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
+        case 3: modal_sources_kernel<3, false><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
+        case 5: modal_sources_kernel<1, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
+        case 6: modal_sources_kernel<2, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
+        case 7: modal_sources_kernel<3, true><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, scale, out, reset); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_cell_records(const GridDims &g, const double *sigma_t, const double *sigma_s, const double *phi,
-                                double *out, cudaStream_t s) {
+                                double *out, int *reset, cudaStream_t s) {
     const int b = blocks_for((size_t)g.nx * g.ny * cell_record_doubles(g.P));
     switch (g.P) {
-        case 1: cell_records_kernel<1><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
-        case 2: cell_records_kernel<2><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
-        case 3: cell_records_kernel<3><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out); break;
+        case 1: cell_records_kernel<1><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out, reset); break;
+        case 2: cell_records_kernel<2><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out, reset); break;
+        case 3: cell_records_kernel<3><<<b, 256, 0, s>>>(g, sigma_t, sigma_s, phi, out, reset); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce_modal_partials(const GridDims &g, const double *part, const int slot_begin[5], size_t stride,
-                                         bool adjoint, const double *minuend, double *phi, cudaStream_t s) {
+                                         bool adjoint, const double *minuend, const double *sigma_s, double *phi,
+                                         cudaStream_t s) {
     SlotBounds sb;
     for (int k = 0; k < 5; ++k) sb.b[k] = slot_begin[k];
     const int b = blocks_for((size_t)(g.nx + 2) * (g.ny + 2));
     switch (g.P + (adjoint ? 4 : 0)) {
-        case 1: reduce_modal_partials_kernel<1, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
-        case 2: reduce_modal_partials_kernel<2, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
-        case 3: reduce_modal_partials_kernel<3, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
-        case 5: reduce_modal_partials_kernel<1, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
-        case 6: reduce_modal_partials_kernel<2, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
-        case 7: reduce_modal_partials_kernel<3, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, phi); break;
+        case 1: reduce_modal_partials_kernel<1, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
+        case 2: reduce_modal_partials_kernel<2, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
+        case 3: reduce_modal_partials_kernel<3, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
+        case 5: reduce_modal_partials_kernel<1, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
+        case 6: reduce_modal_partials_kernel<2, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
+        case 7: reduce_modal_partials_kernel<3, true><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

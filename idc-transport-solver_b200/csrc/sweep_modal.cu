@@ -25,9 +25,10 @@ using modal::prefetch_depth;
 // x' is the sign-flipped ghost source, and the traces are packed modal (Wp h) unless MODAL is false.
 template <int P, bool MODAL>
 __global__ void inflow_traces_kernel(const double *src, const double *xi, const double *eta, int nx, int ny, int nq,
-                                     double *out) {
+                                     double *out, int *reset) {
     constexpr int N = P * P;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx == 0 && reset) *reset = 0;
     if (idx >= (size_t)(nx + ny) * nq) return;
     const int k = (int)(idx / nq), q = (int)(idx % nq);
     const bool xneg = xi[q] < 0, yneg = eta[q] < 0;
@@ -165,11 +166,11 @@ cudaError_t occ_t(int seg, int threads, size_t smem, int *n) {
 
 template <int P, bool MODAL>
 cudaError_t inflow_t(const double *src, const double *xi, const double *eta, int nx, int ny, int nq, double *out,
-                     cudaStream_t stream) {
+                     int *reset, cudaStream_t stream) {
     const size_t n = (size_t)(nx + ny) * nq;
     const int block = 128;
     inflow_traces_kernel<P, MODAL><<<(unsigned)((n + block - 1) / block), block, 0, stream>>>(src, xi, eta, nx, ny,
-                                                                                             nq, out);
+                                                                                             nq, out, reset);
     return cudaGetLastError();
 }
 
@@ -297,14 +298,14 @@ cudaError_t sweep_modal_occupancy(int P, int precision, int seg, int threads, si
 }
 
 cudaError_t launch_inflow_traces(int P, bool modal, const double *src, const double *xi, const double *eta, int nx,
-                                 int ny, int nq, double *out, cudaStream_t stream) {
+                                 int ny, int nq, double *out, int *reset, cudaStream_t stream) {
     switch (P) {
-        case 1: return modal ? inflow_t<1, true>(src, xi, eta, nx, ny, nq, out, stream)
-                             : inflow_t<1, false>(src, xi, eta, nx, ny, nq, out, stream);
-        case 2: return modal ? inflow_t<2, true>(src, xi, eta, nx, ny, nq, out, stream)
-                             : inflow_t<2, false>(src, xi, eta, nx, ny, nq, out, stream);
-        case 3: return modal ? inflow_t<3, true>(src, xi, eta, nx, ny, nq, out, stream)
-                             : inflow_t<3, false>(src, xi, eta, nx, ny, nq, out, stream);
+        case 1: return modal ? inflow_t<1, true>(src, xi, eta, nx, ny, nq, out, reset, stream)
+                             : inflow_t<1, false>(src, xi, eta, nx, ny, nq, out, reset, stream);
+        case 2: return modal ? inflow_t<2, true>(src, xi, eta, nx, ny, nq, out, reset, stream)
+                             : inflow_t<2, false>(src, xi, eta, nx, ny, nq, out, reset, stream);
+        case 3: return modal ? inflow_t<3, true>(src, xi, eta, nx, ny, nq, out, reset, stream)
+                             : inflow_t<3, false>(src, xi, eta, nx, ny, nq, out, reset, stream);
         default: return cudaErrorInvalidValue;
     }
 }
