@@ -72,7 +72,8 @@ namespace lane {
 
 constexpr int kMaxWarps = 7;   // compute warps per thread block; the helper warp is the eighth (two per SM sub-partition)
 constexpr int kStages = 6;     // stages in shared memory: a step's inputs are copied this many steps minus one ahead
-constexpr int kRing = 8;       // columns of y traces between two warps of a thread block
+constexpr int kRing = 16;      // columns of y traces between two warps of a thread block: slack that absorbs the warps' jitter
+                               // (B200, sweep kernel with 8 -> 16: 256x256 Q2 S16 630 -> 607 us, 512x512 Q1 S12 716 -> 659)
 constexpr int kMomStride = 34; // doubles per moment index k in the moment buffer (32 lanes + 2: conflict-free sums)
 
 // Degrees 1 and 2 copy a row segment's source dofs to shared memory, and degree 2 its psi back, in 16-byte chunks: lane o
@@ -221,14 +222,15 @@ __device__ __forceinline__ bool poll_on(long long &polls, int *error, long long 
 }
 // The ring whose consumer has read `*consumed` columns has no room for `column`: wait, and return the first column
 // that may not be written yet, or -1.
-__device__ __forceinline__ int wait_for_credit(uint32_t consumed, int column, int *error, long long spin_limit, int lane) {
+__device__ __forceinline__ int wait_for_credit(uint32_t consumed, int column, int *error, long long spin_limit, int lane,
+                                               unsigned sleep_ns) {
     for (long long polls = 0;;) {
         for (int k = 0; k < kReadsPerPoll; ++k) {
             int c = 0;
             if (lane == 0) c = ld_consumed(consumed);
             c = __shfl_sync(kFullMask, c, 0);
             if (column < c + kRing) return c + kRing;
-            __nanosleep(200);
+            __nanosleep(sleep_ns);
         }
         if (!poll_on(polls, error, spin_limit, lane)) return -1;
     }
@@ -260,7 +262,7 @@ __device__ __noinline__ StepWait<P> wait_for_step(uint32_t slot, bool reader, ui
         if (!poll_on(polls, error, spin_limit, lane)) return r;
     }
     if (cout >= credit && cout < nx) {
-        credit = wait_for_credit(consumed, cout, error, spin_limit, lane);
+        credit = wait_for_credit(consumed, cout, error, spin_limit, lane, 20);
         if (credit < 0) return r;
     }
     r.credit = credit;
@@ -304,7 +306,8 @@ __device__ __forceinline__ void feed_ring(const SweepArgs &a, const SweepItem &i
                     go = false;
                 } else {
                     if (c + k >= credit) {
-                        credit = wait_for_credit(consumed, c + k, a.error, a.spin_limit, lane);
+                        credit = wait_for_credit(consumed, c + k, a.error, a.spin_limit, lane, 200);   // (awake, its polls would take a compute
+                                                                                                         // warp's issue slots)
                         if (credit < 0) return;
                     }
                     const uint32_t slot = ring + 8u * (uint32_t)(((c + k) % kRing) * V + lane);
