@@ -36,10 +36,9 @@ Status bad(int code, const std::string &m) {
     return s;
 }
 
-// Default shape: the single problem's default kernel and rule.  FP64: the lane kernel (warps = 0) with 16-wide
-// segments at DG degree 2, else the narrowest segment with the best lane use.  FP32_REFINED: the modal kernel, narrowest best segment, its default warps.
-void default_shape(int P, int precision, int qmax, int *seg, int *wn) {
-    const bool lane = precision == IDC_PREC_FP64;
+// The narrowest segment with the best lane use for up to qmax ordinates per quadrant (at most 16 wide on the lane kernel).
+int narrow_seg(int qmax, bool lane) {
+    int seg = 4;
     double best = -1.0;
     for (int cand : {4, 8, 16, 32}) {
         if (lane && cand == 32) break;
@@ -47,10 +46,17 @@ void default_shape(int P, int precision, int qmax, int *seg, int *wn) {
         const double eff = (double)qmax / (nch * cand);
         if (eff > best + 1e-9) {
             best = eff;
-            *seg = cand;
+            seg = cand;
         }
     }
-    if (lane && P == 3) *seg = 16;
+    return seg;
+}
+
+// Default shape: the single problem's default kernel and rule.  FP64: the lane kernel (warps = 0) with 16-wide
+// segments at DG degree 2, else the narrowest segment with the best lane use.  FP32_REFINED: the modal kernel, narrowest best segment, its default warps.
+void default_shape(int P, int precision, int qmax, int *seg, int *wn) {
+    const bool lane = precision == IDC_PREC_FP64;
+    *seg = lane && P == 3 ? 16 : narrow_seg(qmax, lane);
     *wn = lane ? 0 : sweep_modal_default_wn(P);
 }
 
@@ -64,17 +70,20 @@ int qmax_of(const Context &c) {
 
 Batch::~Batch() { release(); }
 
+void Batch::release_group(Group &g) {
+    cudaFree(g.d_items);
+    cudaFree(g.d_sync);
+    cudaFree(g.d_table);
+    cudaFreeHost(g.h_table);
+    if (g.upload_done) cudaEventDestroy(g.upload_done);
+    for (double *p : g.trace) cudaFree(p);
+    for (double *p : g.phi_part) cudaFree(p);
+    for (double *p : g.inflow) cudaFree(p);
+    if (g.moments) release_group(*g.moments);
+}
+
 void Batch::release() {
-    for (auto &g : groups) {
-        cudaFree(g.d_items);
-        cudaFree(g.d_sync);
-        cudaFree(g.d_table);
-        cudaFreeHost(g.h_table);
-        if (g.upload_done) cudaEventDestroy(g.upload_done);
-        for (double *p : g.trace) cudaFree(p);
-        for (double *p : g.phi_part) cudaFree(p);
-        for (double *p : g.inflow) cudaFree(p);
-    }
+    for (auto &g : groups) release_group(g);
     groups.clear();
 }
 
@@ -308,15 +317,44 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
                 default_shape(P, precision, qmax, &g.seg, &g.wn);
             }
             g.precision = precision;
-            groups.push_back(g);
+            groups.push_back(std::move(g));
         }
         for (auto &g : groups) IDC_TRY(build_group(g, precision));
     }
     IDC_TRY_CUDA(cudaEventRecord(c0.ev0, c0.stream));
-    for (auto &g : groups) IDC_TRY(launch_group(g, srcs, outs, phi_sc, scale, phis, dt, active, peierls));
+    std::vector<Group *> used;
+    for (auto &g : groups) {
+        Group *u = &g;
+        if (peierls && g.wn == 0 && !tuned.count(std::make_pair(g.P, precision))) {
+            // moments-only sweeps have their own default width, as a single problem's (256x256 Q2 S8: 247 us against
+            // 318 with the full sweep's 16-wide segments)
+            int qmax = 0;
+            for (int m : g.members) qmax = std::max(qmax, qmax_of(*members[m]));
+            const int seg = narrow_seg(qmax, true);
+            if (seg != g.seg) {
+                if (!g.moments) {
+                    auto c = std::make_unique<Group>();
+                    c->P = g.P;
+                    c->seg = seg;
+                    c->members = g.members;
+                    g.moments = std::move(c);   // owned before it holds device memory
+                    Status st = build_group(*g.moments, precision);
+                    if (!st.good()) {
+                        release_group(*g.moments);
+                        g.moments.reset();
+                        return st;
+                    }
+                }
+                u = g.moments.get();
+            }
+        }
+        used.push_back(u);
+    }
+    for (Group *g : used) IDC_TRY(launch_group(*g, srcs, outs, phi_sc, scale, phis, dt, active, peierls));
     IDC_TRY_CUDA(cudaEventRecord(c0.ev1, c0.stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(c0.stream));
-    for (auto &g : groups) {
+    for (Group *gp : used) {
+        Group &g = *gp;
         int err = 0;
         IDC_TRY_CUDA(cudaMemcpy(&err, g.d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost));
         if (err != kDevOk) {

@@ -5,6 +5,7 @@
 
 #include <array>
 #include <map>
+#include <memory>
 #include <utility>
 #include <vector>
 
@@ -52,11 +53,13 @@ private:
         std::vector<double *> trace, phi_part, inflow;
         std::vector<size_t> trace_len;
         std::vector<std::array<int, 5>> slot_begin;   // per member: the quadrants' partial-moment slots
+        std::unique_ptr<Group> moments;   // the moments-only sweeps' schedule where their segment width differs
     };
     Status build_group(Group &g, int precision);
     Status launch_group(Group &g, const double *const *srcs, double *const *outs, const double *const *phi_sc,
                         double scale, double *const *phis, double dt, const std::vector<char> *active, bool peierls);
     void release();
+    static void release_group(Group &g);
     // every group launches on the first member's stream, so that one synchronisation and one event pair
     // cover the whole batched sweep
     cudaStream_t stream() const { return members[0]->stream; }
