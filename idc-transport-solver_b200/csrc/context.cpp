@@ -104,7 +104,6 @@ Status Context::init() {
     IDC_TRY_CUDA(cudaEventCreate(&ev0));
     IDC_TRY_CUDA(cudaEventCreate(&ev1));
     IDC_TRY_CUDA(cudaMalloc(&d_scalar_, sizeof(double) * (4 + multidot_scratch_doubles())));   // + dot scratch
-    IDC_TRY_CUDA(cudaMallocHost(&h_pin_, sizeof(double) * 2));
     // IDC_SWEEP_KERNEL=modal|warp|rowsync selects another sweep kernel than the lane-pipelined one
     if (const char *k = std::getenv("IDC_SWEEP_KERNEL")) {
         const std::string v(k);
@@ -849,14 +848,13 @@ Status Context::sweep_host_many(int64_t count, const double *const *srcs, double
 }
 
 Status Context::check_device_error() {
-    IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_ + 1, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    int err = 0;
+    IDC_TRY_CUDA(cudaMemcpyAsync(&err, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
-    return report_device_error();
+    return report_device_error(err);
 }
 
-Status Context::report_device_error() {
-    int err = 0;
-    std::memcpy(&err, h_pin_ + 1, sizeof(int));
+Status Context::report_device_error(int err) {
     if (err != kDevOk) {
         IDC_TRY_CUDA(cudaMemsetAsync(d_sync + 1, 0, sizeof(int), stream));
         if (d_trace)
@@ -1158,11 +1156,14 @@ Status Context::transport_residual_transpose(const double *z, double *y, double 
 Status Context::l2dist(const double *a, const double *b, double *out_host, bool checked) {
     IDC_TRY_CUDA(launch_l2dist2(dims(), a, b, d_scalar_, d_scalar_ + 4, stream));
     launches += 2;
+    if (!h_pin_) IDC_TRY_CUDA(cudaMallocHost(&h_pin_, sizeof(double) * 2));   // (solvers only: a pinned allocation takes a while)
     IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
     if (checked) IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_ + 1, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
     *out_host = std::sqrt(h_pin_[0]);
-    return checked ? report_device_error() : Status::ok();
+    int err = kDevOk;
+    if (checked) std::memcpy(&err, h_pin_ + 1, sizeof(int));
+    return report_device_error(err);
 }
 
 // SISolver::Solve, linear_solvers/Abstract/ImplicitSolver/SISolver.cpp:190-254.  The copy of the

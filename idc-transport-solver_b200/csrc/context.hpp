@@ -57,7 +57,7 @@ public:
     Status transport_residual(const double *psi, const double *phi, double *res);   // (L - S P) psi, phi = P psi
     // |a - b|; checked: and the device error word with it, as check_device_error, in one synchronisation
     Status l2dist(const double *a, const double *b, double *out_host, bool checked = false);
-    Status report_device_error();   // a recorded error: clears it, re-arms the trace buffers, IDC_ERR_TIMEOUT
+    Status report_device_error(int err);   // a recorded error: clears it, re-arms the trace buffers, IDC_ERR_TIMEOUT
     Status source_iteration(const double *src, double *psi_out, double dt, double abs_tol, int64_t max_its,
                             int precision, int64_t *iters, double *err);
     // phi_guess (optional, moment-sized, device): GMRES starts from it instead of zero (reflecting or periodic

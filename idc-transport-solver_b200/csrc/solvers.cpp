@@ -36,6 +36,7 @@ Status bad(int code, const std::string &m) {
 Status Context::dot_host(const double *x, const double *y, size_t n, double *out) {
     IDC_TRY_CUDA(launch_dot(x, y, n, d_scalar_, d_scalar_ + 4, stream));
     launches += 2;
+    if (!h_pin_) IDC_TRY_CUDA(cudaMallocHost(&h_pin_, sizeof(double) * 2));
     IDC_TRY_CUDA(cudaMemcpyAsync(h_pin_, d_scalar_, sizeof(double), cudaMemcpyDeviceToHost, stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(stream));
     *out = h_pin_[0];

@@ -116,41 +116,41 @@ __global__ void cell_records_kernel(GridDims g, const double *__restrict__ sigma
 struct SlotBounds {
     int b[5];
 };
+// Four lanes per cell, one per quadrant: the sums over the slots are chains of loads, and a thread per cell left small
+// grids with a few blocks of them (B200, 64x64 Q1 S8 8.9 us).
 template <int P, bool ADJ>
 __device__ __forceinline__ void reduce_modal_partials(int nx, int ny, const double *__restrict__ part, const SlotBounds &sb,
                                                       size_t stride, const double *__restrict__ minuend,
                                                       const double *__restrict__ sigma_s, double *__restrict__ phi) {
     constexpr int N = P * P;
     const size_t total = (size_t)(nx + 2) * (ny + 2);
-    for (size_t cidx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; cidx < total;
-         cidx += (size_t)gridDim.x * blockDim.x) {
+    const int k = threadIdx.x & 3, lane = threadIdx.x & 31;
+    const bool xn = k >= 2, yn = (k & 1) != 0;
+    // whole warps stay together: 8 cells a turn
+    for (size_t c0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x - lane) / 4; c0 < total;
+         c0 += (size_t)gridDim.x * blockDim.x / 4) {
+        const size_t cidx = c0 + lane / 4;
         const int i = (int)(cidx / (ny + 2)), j = (int)(cidx % (ny + 2));
-        double acc[N];
-#pragma unroll
-        for (int m = 0; m < N; ++m) acc[m] = 0.0;
         const bool interior = i >= 1 && i <= nx && j >= 1 && j <= ny;
-        if (interior) {
-            for (int k = 0; k < 4; ++k) {
-                if (sb.b[k + 1] == sb.b[k]) continue;
-                double M[N], x[N];
+        double M[N], x[N];
 #pragma unroll
-                for (int m = 0; m < N; ++m) M[m] = 0.0;
-                for (int sl = sb.b[k]; sl < sb.b[k + 1]; ++sl)
+        for (int m = 0; m < N; ++m) M[m] = 0.0;
+        if (interior)
+            for (int sl = sb.b[k]; sl < sb.b[k + 1]; ++sl)
 #pragma unroll
-                    for (int m = 0; m < N; ++m) M[m] += part[(size_t)sl * stride + cidx * N + m];
-                modal_backward<P, false, false, double, ADJ>(x, M);
-                const bool xn = k >= 2, yn = (k & 1) != 0;
-#pragma unroll
-                for (int m = 0; m < N; ++m) {
-                    const int d = m / P, e = m % P;
-                    acc[m] += (((d & 1) && xn) != ((e & 1) && yn)) ? -x[m] : x[m];
-                }
-            }
-        }
+                for (int m = 0; m < N; ++m) M[m] += part[(size_t)sl * stride + cidx * N + m];
+        modal_backward<P, false, false, double, ADJ>(x, M);
 #pragma unroll
         for (int m = 0; m < N; ++m) {
-            const double v = sigma_s && interior ? sigma_s[cidx] / (4.0 * M_PI) * acc[m] : acc[m];
-            phi[cidx * N + m] = minuend ? minuend[cidx * N + m] - v : v;
+            const int d = m / P, e = m % P;
+            const double own = (((d & 1) && xn) != ((e & 1) && yn)) ? -x[m] : x[m];
+            double acc = 0.0;   // the quadrants in order
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc += __shfl_sync(kFullMask, own, (lane & ~3) + q);
+            if (k == m % 4 && cidx < total) {
+                const double v = sigma_s && interior ? sigma_s[cidx] / (4.0 * M_PI) * acc : acc;
+                phi[cidx * N + m] = minuend ? minuend[cidx * N + m] - v : v;
+            }
         }
     }
 }
@@ -254,7 +254,7 @@ cudaError_t launch_reduce_modal_partials(const GridDims &g, const double *part, 
                                          cudaStream_t s) {
     SlotBounds sb;
     for (int k = 0; k < 5; ++k) sb.b[k] = slot_begin[k];
-    const int b = blocks_for((size_t)(g.nx + 2) * (g.ny + 2));
+    const int b = blocks_for((size_t)(g.nx + 2) * (g.ny + 2) * 4);
     switch (g.P + (adjoint ? 4 : 0)) {
         case 1: reduce_modal_partials_kernel<1, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
         case 2: reduce_modal_partials_kernel<2, false><<<b, 256, 0, s>>>(g, part, sb, stride, minuend, sigma_s, phi); break;
