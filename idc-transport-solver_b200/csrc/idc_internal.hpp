@@ -1,6 +1,7 @@
 // Internal declarations shared by the CUDA kernels, the C++ host layer and the C ABI.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cstddef>
 #include <functional>
@@ -89,6 +90,25 @@ struct SweepArgs {
 
 // Doubles of a cell's record: N moments, sigma_t, rounded up to whole 16-byte words.
 __host__ __device__ constexpr int cell_record_doubles(int P) { return (P * P + 2) / 2 * 2; }
+
+constexpr int kMaxBlockSmem = 227 << 10;   // sm_100: shared memory a thread block may have, static and dynamic
+
+// Lets a kernel be launched with all the dynamic shared memory a thread block may have.  The limit is the kernel's, and
+// contexts in other host threads launch the same kernel with other sizes: every caller sets the same value, so none finds
+// it lowered between setting it and launching.
+template <auto Kernel>
+cudaError_t allow_dynamic_smem() {
+    static std::atomic<int> limit{0};   // (a property of the compiled kernel)
+    int n = limit.load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaFuncAttributes at;
+        cudaError_t e = cudaFuncGetAttributes(&at, Kernel);
+        if (e != cudaSuccess) return e;
+        n = kMaxBlockSmem - (int)at.sharedSizeBytes;
+        limit.store(n, std::memory_order_relaxed);
+    }
+    return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
+}
 
 // Launch geometry picked by the host (autotuner or defaults).
 struct SweepTiling {

@@ -201,8 +201,8 @@ size_t sweep_smem_bytes(int P, int R, int G) {
 
 template <int P, int MODE>
 static cudaError_t launch_one(const SweepArgs &args, int grid, int block, size_t smem, cudaStream_t stream) {
-    auto kern = sweep_kernel<P, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kern = sweep_kernel<P, MODE>;
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     kern<<<grid, block, smem, stream>>>(args);
     return cudaGetLastError();
@@ -210,8 +210,8 @@ static cudaError_t launch_one(const SweepArgs &args, int grid, int block, size_t
 
 template <int P, int MODE>
 static cudaError_t occ_one(int block, size_t smem, int *n) {
-    auto kern = sweep_kernel<P, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kern = sweep_kernel<P, MODE>;
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kern, block, smem);
 }

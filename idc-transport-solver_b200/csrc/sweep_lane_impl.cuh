@@ -785,9 +785,9 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1)
 
 template <int P, int SEG, bool ADJ, bool SRC2, bool PHI = false, typename TC = double>
 cudaError_t launch(const SweepArgs &args, int grid, cudaStream_t stream) {
-    auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, PHI, TC, false>;
+    constexpr auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, PHI, TC, false>;
     const size_t smem = block_smem_bytes(P, SEG, SRC2, PHI, args.wn);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     kern<<<grid, (args.wn + 1) * 32, smem, stream>>>(args, nullptr);
     return cudaGetLastError();
@@ -797,9 +797,9 @@ cudaError_t launch(const SweepArgs &args, int grid, cudaStream_t stream) {
 // problem)
 template <int P, int SEG, bool PHI>
 cudaError_t launch_batched(const SweepArgs &args, const SweepArgs *table, int grid, cudaStream_t stream) {
-    auto kern = sweep_lane_kernel<P, SEG, false, false, PHI, double, true>;
+    constexpr auto kern = sweep_lane_kernel<P, SEG, false, false, PHI, double, true>;
     const size_t smem = block_smem_bytes(P, SEG, false, PHI, args.wn);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     kern<<<grid, (args.wn + 1) * 32, smem, stream>>>(args, table);
     return cudaGetLastError();
@@ -808,18 +808,18 @@ cudaError_t launch_batched(const SweepArgs &args, const SweepArgs *table, int gr
 // (of the full sweep: the moments-only instance needs less)
 template <int P, int SEG>
 cudaError_t occupancy_batched(int warps, int *blocks_per_sm) {
-    auto kern = sweep_lane_kernel<P, SEG, false, false, false, double, true>;
+    constexpr auto kern = sweep_lane_kernel<P, SEG, false, false, false, double, true>;
     const size_t smem = block_smem_bytes(P, SEG, false, false, warps);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, (warps + 1) * 32, smem);
 }
 
 template <int P, int SEG, bool ADJ, bool SRC2>
 cudaError_t occupancy(int warps, int *blocks_per_sm) {
-    auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, false, double, false>;
+    constexpr auto kern = sweep_lane_kernel<P, SEG, ADJ, SRC2, false, double, false>;
     const size_t smem = block_smem_bytes(P, SEG, SRC2, false, warps);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, (warps + 1) * 32, smem);
 }

@@ -685,36 +685,36 @@ __global__ void __launch_bounds__(max_warps(P) * 32, 1) sweep_modal_kernel(const
     }
 }
 
+template <auto Kernel>
+cudaError_t launch_kernel(int P, const SweepArgs &args, const SweepArgs *table, int grid, size_t smem, cudaStream_t stream) {
+    cudaError_t e = allow_dynamic_smem<Kernel>();
+    if (e != cudaSuccess) return e;
+    Kernel<<<grid, cta_warps(P, args.wn) * 32, smem, stream>>>(args, table);
+    return cudaGetLastError();
+}
+
 template <int P, int MODE, int SEG, bool ADJ>
 cudaError_t launch_seg(const SweepArgs &args, int grid, size_t smem, cudaStream_t stream) {
     // the second source has its own instantiation (forward, FP64 and refined precision), so the other
     // launches run the kernel without it
-    auto kern = sweep_modal_kernel<P, MODE, SEG, ADJ, false>;
     if constexpr (!ADJ && MODE != 2) {
-        if (args.src2) kern = sweep_modal_kernel<P, MODE, SEG, false, false, true>;
+        if (args.src2) return launch_kernel<sweep_modal_kernel<P, MODE, SEG, false, false, true>>(P, args, nullptr, grid, smem, stream);
     } else {
         if (args.src2) return cudaErrorInvalidValue;
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, cta_warps(P, args.wn) * 32, smem, stream>>>(args, nullptr);
-    return cudaGetLastError();
+    return launch_kernel<sweep_modal_kernel<P, MODE, SEG, ADJ, false>>(P, args, nullptr, grid, smem, stream);
 }
 
 template <int P, int MODE, int SEG>
 cudaError_t launch_seg_batched(const SweepArgs &launch, const SweepArgs *table, int grid, size_t smem,
                                cudaStream_t stream) {
-    auto kern = sweep_modal_kernel<P, MODE, SEG, false, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, cta_warps(P, launch.wn) * 32, smem, stream>>>(launch, table);
-    return cudaGetLastError();
+    return launch_kernel<sweep_modal_kernel<P, MODE, SEG, false, true>>(P, launch, table, grid, smem, stream);
 }
 
 template <int P, int MODE, int SEG, bool ADJ>
 cudaError_t occ_seg(int threads, size_t smem, int *n) {
-    auto kern = sweep_modal_kernel<P, MODE, SEG, ADJ, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kern = sweep_modal_kernel<P, MODE, SEG, ADJ, false>;
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kern, threads, smem);
 }

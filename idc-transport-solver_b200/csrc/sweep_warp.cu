@@ -468,8 +468,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) sweep_warp_kernel(const Swe
 
 template <int P, int MODE>
 cudaError_t launch_t(const SweepArgs &args, int grid, size_t smem, cudaStream_t stream) {
-    auto kern = sweep_warp_kernel<P, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kern = sweep_warp_kernel<P, MODE>;
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     kern<<<grid, (args.wn + 1) * 32, smem, stream>>>(args);
     return cudaGetLastError();
@@ -477,8 +477,8 @@ cudaError_t launch_t(const SweepArgs &args, int grid, size_t smem, cudaStream_t 
 
 template <int P, int MODE>
 cudaError_t occ_t(int threads, size_t smem, int *n) {
-    auto kern = sweep_warp_kernel<P, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr auto kern = sweep_warp_kernel<P, MODE>;
+    cudaError_t e = allow_dynamic_smem<kern>();
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kern, threads, smem);
 }
