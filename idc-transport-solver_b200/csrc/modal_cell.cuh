@@ -122,18 +122,8 @@ __device__ __forceinline__ float recip_fast(float x) {
     return r;
 }
 
-// 1/x for positive normal x by one cubic Newton-Raphson step (e = 1 - x y, y (1 + e + e^2)) from the hardware
-// approximation (20 bits): e^3 < 2^-60, so the result is within an ulp of 1/x.  No branch, unlike the correctly rounded
-// reciprocal, whose range checks split the sweep's basic block (B200, moments-only sweep: 256x256 Q2 S16 347 -> 326 us).
-__device__ __forceinline__ double recip_newton(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    e = fma(e, e, e);
-    return fma(y, e, y);
-}
-
-// Reciprocals of the cell's |D|^2 (positive reals).  FP64: one reciprocal of their product and a product chain (Montgomery's simultaneous inversion); the product of the five |D|^2 of
+// Reciprocals of the cell's |D|^2 (positive reals).  FP64: one correctly rounded reciprocal of their
+// product and a product chain (Montgomery's simultaneous inversion); the product of the five |D|^2 of
 // P = 3 stays finite for |D| below 1e30.  FP32: one hardware reciprocal each.
 template <int K>
 __device__ __forceinline__ void batch_recip(double (&v)[K]) {
@@ -141,7 +131,7 @@ __device__ __forceinline__ void batch_recip(double (&v)[K]) {
     pre[0] = v[0];
 #pragma unroll
     for (int k = 1; k < K; ++k) pre[k] = pre[k - 1] * v[k];
-    double inv = recip_newton(pre[K - 1]);
+    double inv = __drcp_rn(pre[K - 1]);
 #pragma unroll
     for (int k = K - 1; k > 0; --k) {
         const double vk = v[k];
