@@ -54,11 +54,6 @@ int fail(int code, const char *msg) {
     catch (const std::bad_alloc &) { return fail(IDC_ERR_NOMEM, "host allocation failed"); } \
     catch (...) { return fail(IDC_ERR_CUDA, "unexpected exception in idcsweep"); }
 
-// The solvers work on the caller's device array from their first microseconds on, on the context's own non-blocking
-// stream: what the caller has queued on the legacy default stream to fill it (a copy that the call follows at once) is
-// finished first.
-cudaError_t caller_ready() { return cudaStreamSynchronize(cudaStreamLegacy); }
-
 bool valid_loc(int loc) { return loc == IDC_LOC_HOST || loc == IDC_LOC_DEVICE; }
 
 }  // namespace
@@ -93,6 +88,8 @@ int adjoint_time_abi(const char *name, idc_ctx *ctx, const double *psi0, const d
         d_gs = dsigma_s ? c.phi_buf(13) : nullptr;
         d_gq = dsource ? c.phi_buf(14) : nullptr;
         d_p0 = dpsi0 ? c.psi_buf(2) : nullptr;
+    } else {
+        ABI_TRY(c.after_caller());
     }
     ABI_TRY_CUDA(cudaMemcpyAsync(d_det, detector, sizeof(double) * c.phi_len(), in, c.stream));
     ABI_TRY_CUDA(idc::launch_zero_ghost_phi(c.dims(), d_det, c.stream));
@@ -211,6 +208,7 @@ int idc_sweep(idc_ctx *ctx, double *psi_inout, double dt, double *phi_out, int p
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.sweep(psi_inout, psi_inout, dt, phi_out, precision));
         ABI_TRY(c.check_device_error());
     } else {
@@ -241,6 +239,7 @@ int idc_sweep_out(idc_ctx *ctx, const double *source, double *result, double dt,
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.sweep(source, result, dt, phi_out, precision));
         ABI_TRY(c.check_device_error());
     } else {
@@ -275,6 +274,7 @@ int idc_sweep_out_many(idc_ctx *ctx, int64_t count, const double *const *sources
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         for (int64_t k = 0; k < count; ++k) ABI_TRY(c.sweep(sources[k], results[k], dt, phi_out ? phi_out[k] : nullptr, precision));
         ABI_TRY(c.check_device_error());
     } else {
@@ -294,6 +294,7 @@ int idc_pmv(idc_ctx *ctx, double alpha, double beta, const double *psi, double *
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.pmv(alpha, beta, psi, phi));
     } else {
         ABI_TRY(c.ensure_psi_buffers(1));
@@ -317,6 +318,7 @@ int idc_smv(idc_ctx *ctx, double alpha, double beta, const double *phi, double *
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.smv(alpha, beta, phi, psi));
     } else {
         ABI_TRY(c.ensure_psi_buffers(1));
@@ -341,6 +343,7 @@ int idc_lmv(idc_ctx *ctx, double alpha, double beta, const double *x, double *y,
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.lmv(alpha, beta, x, y));
     } else {
         ABI_TRY(c.ensure_psi_buffers(2));
@@ -367,7 +370,7 @@ int idc_source_iteration(idc_ctx *ctx, double *source_inout, double dt, double a
     double *d_src = c.psi_buf(1), *d_psi = c.psi_buf(0);
     const cudaMemcpyKind in = loc == IDC_LOC_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     const cudaMemcpyKind out = loc == IDC_LOC_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    if (loc == IDC_LOC_DEVICE) ABI_TRY_CUDA(caller_ready());
+    if (loc == IDC_LOC_DEVICE) ABI_TRY(c.after_caller());
     ABI_TRY_CUDA(cudaMemcpyAsync(d_src, source_inout, sizeof(double) * c.psi_len(), in, c.stream));
     // psi starts as the source so that its ghost cells hold the inflow values (SISolver copies
     // Interior|Boundary from the source every iteration, SISolver.cpp:226)
@@ -400,7 +403,7 @@ int idc_gmres_solve(idc_ctx *ctx, double *source_inout, double dt, double abs_to
         d_psi = c.psi_buf(0);
         ABI_TRY_CUDA(cudaMemcpyAsync(d_psi, source_inout, sizeof(double) * c.psi_len(), cudaMemcpyHostToDevice, c.stream));
     } else {
-        ABI_TRY_CUDA(caller_ready());
+        ABI_TRY(c.after_caller());
     }
     int64_t its = 0;
     double res = 0;
@@ -442,6 +445,8 @@ int idc_idc_integrate(idc_ctx *ctx, double *psi_inout, const double *source, dou
                                      c.stream));
         d_psi = c.psi_buf(0);
         d_src = c.psi_buf(1);
+    } else {
+        ABI_TRY(c.after_caller());
     }
     int64_t n_sweeps = 0;
     idc::Status st = c.idc_integrate(d_psi, d_src, dt, steps, num_nodes, num_corrections, scattering, precision,
@@ -463,6 +468,7 @@ int idc_sweep_fused(idc_ctx *ctx, const double *source, double *result, double d
     idc::Context &c = ctx->impl;
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
+    ABI_TRY(c.after_caller());
     ABI_TRY(c.sweep(source, result, dt, phi_out, precision, phi_scatter, scatter_scale));
     ABI_TRY(c.check_device_error());
     float ms = 0.f;
@@ -485,6 +491,7 @@ int idc_autotune(idc_ctx *ctx, const double *source, double dt, int precision, i
     idc::Context &c = ctx->impl;
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     int s = 0, w = 0;
+    ABI_TRY(c.after_caller());
     ABI_TRY(c.autotune(source, dt, precision, &s, &w));
     if (seg) *seg = s;
     if (warps) *warps = w;
@@ -513,6 +520,7 @@ int idc_batch_sweep(idc_batch *b, const double *const *sources, double *const *r
                     double dt, int precision) {
     ABI_GUARD_BEGIN
     if (!b) return fail(IDC_ERR_ARG, "idc_batch_sweep: null batch");
+    ABI_TRY(b->impl.after_caller());
     ABI_TRY(b->impl.sweep(sources, results, nullptr, 1.0, phi_out, dt, precision));
     return IDC_OK;
     ABI_GUARD_END
@@ -521,6 +529,7 @@ int idc_batch_sweep(idc_batch *b, const double *const *sources, double *const *r
 int idc_batch_autotune(idc_batch *b, const double *const *sources, double *const *results, double dt, int precision) {
     ABI_GUARD_BEGIN
     if (!b) return fail(IDC_ERR_ARG, "idc_batch_autotune: null batch");
+    ABI_TRY(b->impl.after_caller());
     ABI_TRY(b->impl.autotune(sources, results, dt, precision));
     return IDC_OK;
     ABI_GUARD_END
@@ -554,6 +563,7 @@ int idc_batch_gmres_solve(idc_batch *b, double *const *psi_inout, double dt, dou
     ABI_GUARD_BEGIN
     if (!b || !psi_inout) return fail(IDC_ERR_ARG, "idc_batch_gmres_solve: null argument");
     if (max_its < 0 || !(abs_tol >= 0)) return fail(IDC_ERR_ARG, "idc_batch_gmres_solve: bad tolerance");
+    ABI_TRY(b->impl.after_caller());
     ABI_TRY(b->impl.gmres_solve(psi_inout, dt, abs_tol, restart, max_its, precision, iters, final_resids));
     return IDC_OK;
     ABI_GUARD_END
@@ -574,6 +584,7 @@ int idc_sweep_adjoint(idc_ctx *ctx, const double *source, double *result, double
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
     if (loc == IDC_LOC_DEVICE) {
+        ABI_TRY(c.after_caller());
         ABI_TRY(c.sweep(source, result, dt, moments_out, precision, nullptr, 1.0, true));
         ABI_TRY(c.check_device_error());
     } else {
@@ -618,6 +629,8 @@ int idc_adjoint_grad(idc_ctx *ctx, const double *psi, const double *detector, do
         d_gt = dsigma_t ? c.phi_buf(11) : nullptr;   // sigma-sized results fit a moment-sized buffer
         d_gs = dsigma_s ? c.phi_buf(12) : nullptr;
         d_gq = dsource ? c.phi_buf(13) : nullptr;
+    } else {
+        ABI_TRY(c.after_caller());
     }
     ABI_TRY_CUDA(cudaMemcpyAsync(d_det, detector, sizeof(double) * c.phi_len(), in, c.stream));
     ABI_TRY_CUDA(idc::launch_zero_ghost_phi(c.dims(), d_det, c.stream));
@@ -676,6 +689,7 @@ int idc_lmv_transpose(idc_ctx *ctx, double alpha, double beta, const double *x, 
     if (loc != IDC_LOC_DEVICE) return fail(IDC_ERR_ARG, "idc_lmv_transpose: device arrays only");
     idc::Context &c = ctx->impl;
     if (!c.have_ordinates || !c.have_sigma) return fail(IDC_ERR_STATE, "idc_lmv_transpose before ordinates and sigma");
+    ABI_TRY(c.after_caller());
     ABI_TRY(c.lmv_transpose(alpha, beta, x, y));
     ABI_TRY_CUDA(cudaStreamSynchronize(c.stream));
     return IDC_OK;

@@ -15,6 +15,7 @@ class Batch {
 public:
     ~Batch();
     Status add(Context *c);
+    Status after_caller() { return members.empty() ? Status::ok() : members[0]->after_caller(); }   // (all groups' stream)
     // per problem p (arrays indexed like `members`, entries nullable): outs[p] <- L^{-1}(srcs[p] +
     // scale phi_sc[p]), phis[p] <- P outs[p]; device pointers.  phi_sc[p] holds the scattering moments
     // sigma_s phi / (4 pi) per cell, S phi without the ordinate broadcast: launch_cell_records for members on the

@@ -87,6 +87,7 @@ Context::~Context() {
     if (copy_out) cudaStreamDestroy(copy_out);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    if (ev_caller) cudaEventDestroy(ev_caller);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -103,6 +104,7 @@ Status Context::init() {
     IDC_TRY_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     IDC_TRY_CUDA(cudaEventCreate(&ev0));
     IDC_TRY_CUDA(cudaEventCreate(&ev1));
+    IDC_TRY_CUDA(cudaEventCreateWithFlags(&ev_caller, cudaEventDisableTiming));
     IDC_TRY_CUDA(cudaMalloc(&d_scalar_, sizeof(double) * (4 + multidot_scratch_doubles())));   // + dot scratch
     // IDC_SWEEP_KERNEL=modal|warp|rowsync selects another sweep kernel than the lane-pipelined one
     if (const char *k = std::getenv("IDC_SWEEP_KERNEL")) {
@@ -489,6 +491,21 @@ Status Context::set_sigma(const double *sigma_t, const double *sigma_s, int loc)
     // (the copies above may still be under way when they return, and the context's stream does not wait for theirs)
     IDC_TRY_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     have_sigma = true;
+    return Status::ok();
+}
+
+Status Context::after_caller() {
+    IDC_TRY_CUDA(cudaSetDevice(device));
+    // (while a blocking stream of this process is being captured the default stream takes no work, and asking it is an error)
+    cudaStreamCaptureStatus capture;
+    const cudaError_t can = cudaStreamIsCapturing(cudaStreamLegacy, &capture);
+    if (can == cudaErrorStreamCaptureImplicit) {
+        (void)cudaGetLastError();
+        return Status::ok();
+    }
+    IDC_TRY_CUDA(can);
+    IDC_TRY_CUDA(cudaEventRecord(ev_caller, cudaStreamLegacy));
+    IDC_TRY_CUDA(cudaStreamWaitEvent(stream, ev_caller, 0));
     return Status::ok();
 }
 

@@ -38,6 +38,9 @@ public:
     Status autotune(const double *src, double dt, int precision, int *seg_out, int *wn_out);
 
     // ---- operators on device pointers ----
+    // The stream waits for what the caller has queued on the legacy default stream (the library's streams are
+    // non-blocking ones): every call that works on the caller's device arrays begins with this.
+    Status after_caller();
     // Sweep: out <- L^{-1} (src [+ scale * S phi_scatter]); phi (nullable) <- P out.  src may equal out.
     // src2 (modal kernel, forward): the source is src + src2_scale * src2 on interior cells, combined by the
     // sweep's aux warps (or, when its stages do not fit in shared memory, by a kernel into a scratch array)
@@ -130,7 +133,7 @@ public:
     int device = 0;
     int num_sms = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_caller = nullptr;
 
     int64_t nq = 0;
     int64_t quad[5] = {0, 0, 0, 0, 0};

@@ -17,7 +17,10 @@
  * Pointers marked "loc" are host pointers when loc == IDC_LOC_HOST (the library copies them to and from
  * its own device buffers inside the call) and device pointers on the context's GPU when
  * loc == IDC_LOC_DEVICE (the call works on them in place).  Calls are synchronous: when one returns, its
- * results are in place.  A context is not re-entrant: use one context per host thread.
+ * results are in place.  The library works on streams of its own: a call on device arrays waits for what was
+ * queued before it on the legacy default stream of the context's GPU, and on blocking streams, to which that
+ * one is ordered (a copy that fills the array, say); work queued on non-blocking streams has to be finished
+ * when the call is made.  A context is not re-entrant: use one context per host thread.
  */
 #ifndef IDCSWEEP_H
 #define IDCSWEEP_H
