@@ -162,9 +162,9 @@ Status Batch::build_group(Group &g, int precision) {
     g.items_per_rb = ipr;
     IDC_TRY_CUDA(cudaSetDevice(c0.device));
     IDC_TRY_CUDA(cudaMalloc(&g.d_items, sizeof(SweepItem) * items.size()));
-    IDC_TRY_CUDA(cudaMemcpy(g.d_items, items.data(), sizeof(SweepItem) * items.size(), cudaMemcpyHostToDevice));
+    IDC_TRY(c0.upload(g.d_items, items.data(), sizeof(SweepItem) * items.size()));
     IDC_TRY_CUDA(cudaMalloc(&g.d_sync, sizeof(int) * 2));
-    IDC_TRY_CUDA(cudaMemset(g.d_sync, 0, sizeof(int) * 2));
+    IDC_TRY_CUDA(cudaMemsetAsync(g.d_sync, 0, sizeof(int) * 2, c0.stream));
     IDC_TRY_CUDA(cudaMalloc(&g.d_table, sizeof(SweepArgs) * g.members.size()));
     IDC_TRY_CUDA(cudaMallocHost(&g.h_table, sizeof(SweepArgs) * g.members.size()));
     IDC_TRY_CUDA(cudaEventCreateWithFlags(&g.upload_done, cudaEventDisableTiming));
@@ -358,7 +358,7 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
         int err = 0;
         IDC_TRY_CUDA(cudaMemcpy(&err, g.d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost));
         if (err != kDevOk) {
-            IDC_TRY_CUDA(cudaMemset(g.d_sync + 1, 0, sizeof(int)));
+            IDC_TRY_CUDA(cudaMemsetAsync(g.d_sync + 1, 0, sizeof(int), c0.stream));
             for (size_t m = 0; m < g.members.size(); ++m)
                 IDC_TRY_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long *>(g.trace[m]), g.trace_len[m],
                                              kTraceSentinel, c0.stream));

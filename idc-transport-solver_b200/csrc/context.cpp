@@ -141,9 +141,9 @@ Status Context::set_ordinates(int64_t nq_in, const double *xi, const double *eta
     IDC_TRY_CUDA(cudaMalloc(&d_xi, sizeof(double) * nq_in));
     IDC_TRY_CUDA(cudaMalloc(&d_eta, sizeof(double) * nq_in));
     IDC_TRY_CUDA(cudaMalloc(&d_w, sizeof(double) * nq_in));
-    IDC_TRY_CUDA(cudaMemcpy(d_xi, xi, sizeof(double) * nq_in, cudaMemcpyHostToDevice));
-    IDC_TRY_CUDA(cudaMemcpy(d_eta, eta, sizeof(double) * nq_in, cudaMemcpyHostToDevice));
-    IDC_TRY_CUDA(cudaMemcpy(d_w, w, sizeof(double) * nq_in, cudaMemcpyHostToDevice));
+    IDC_TRY(upload(d_xi, xi, sizeof(double) * nq_in));
+    IDC_TRY(upload(d_eta, eta, sizeof(double) * nq_in));
+    IDC_TRY(upload(d_w, w, sizeof(double) * nq_in));
     if (nq_in != nq) {
         // psi-sized buffers (and the unweighted-sum weights) depend on nq
         for (auto *v : {&psi_bufs_, &idc_psi_, &transient_bufs_, &adj_idc_bufs_}) {
@@ -196,7 +196,7 @@ Status Context::update_reflect_map() {
     cudaFree(d_rmap);
     d_rmap = nullptr;
     IDC_TRY_CUDA(cudaMalloc(&d_rmap, sizeof(int) * map.size()));
-    IDC_TRY_CUDA(cudaMemcpy(d_rmap, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice));
+    IDC_TRY(upload(d_rmap, map.data(), sizeof(int) * map.size()));
     return Status::ok();
 }
 
@@ -465,6 +465,7 @@ Status Context::set_sigma(const double *sigma_t, const double *sigma_s, int loc)
     if (!d_sigma_t) IDC_TRY_CUDA(cudaMalloc(&d_sigma_t, sizeof(double) * sig_len()));
     if (!d_sigma_s) IDC_TRY_CUDA(cudaMalloc(&d_sigma_s, sizeof(double) * sig_len()));
     const cudaMemcpyKind kind = loc == IDC_LOC_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
+    if (loc == IDC_LOC_DEVICE) IDC_TRY(after_caller());
     if (high_order_sigma()) {   // Legendre moments [cell][u][v] of both cross sections
         const size_t nm = sig_len() * N, nt = sig_len() * N * N;
         if (!d_sig_mom_) IDC_TRY_CUDA(cudaMalloc(&d_sig_mom_, sizeof(double) * nm));
@@ -483,14 +484,19 @@ Status Context::set_sigma(const double *sigma_t, const double *sigma_s, int loc)
         have_sigma = true;
         return Status::ok();
     }
-    IDC_TRY_CUDA(cudaMemcpy(d_sigma_t, sigma_t, sizeof(double) * sig_len(), kind));
+    IDC_TRY_CUDA(cudaMemcpyAsync(d_sigma_t, sigma_t, sizeof(double) * sig_len(), kind, stream));
     if (sigma_s)
-        IDC_TRY_CUDA(cudaMemcpy(d_sigma_s, sigma_s, sizeof(double) * sig_len(), kind));
+        IDC_TRY_CUDA(cudaMemcpyAsync(d_sigma_s, sigma_s, sizeof(double) * sig_len(), kind, stream));
     else
-        IDC_TRY_CUDA(cudaMemset(d_sigma_s, 0, sizeof(double) * sig_len()));
-    // (the copies above may still be under way when they return, and the context's stream does not wait for theirs)
-    IDC_TRY_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        IDC_TRY_CUDA(cudaMemsetAsync(d_sigma_s, 0, sizeof(double) * sig_len(), stream));
+    IDC_TRY_CUDA(cudaStreamSynchronize(stream));
     have_sigma = true;
+    return Status::ok();
+}
+
+Status Context::upload(void *dst, const void *src, size_t bytes) {
+    IDC_TRY_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
+    IDC_TRY_CUDA(cudaStreamSynchronize(stream));
     return Status::ok();
 }
 
@@ -592,7 +598,7 @@ Status Context::ensure_phi_buffers(int count) {
     while ((int)phi_bufs_.size() < count) {
         double *p = nullptr;
         IDC_TRY_CUDA(cudaMalloc(&p, sizeof(double) * phi_len()));
-        IDC_TRY_CUDA(cudaMemset(p, 0, sizeof(double) * phi_len()));
+        IDC_TRY_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * phi_len(), stream));
         phi_bufs_.push_back(p);
     }
     return Status::ok();
@@ -769,17 +775,20 @@ Status Context::build_schedule(int precision) {
     cudaFree(d_items);
     d_items = nullptr;
     IDC_TRY_CUDA(cudaMalloc(&d_items, sizeof(SweepItem) * items.size()));
-    IDC_TRY_CUDA(cudaMemcpy(d_items, items.data(), sizeof(SweepItem) * items.size(), cudaMemcpyHostToDevice));
+    IDC_TRY(upload(d_items, items.data(), sizeof(SweepItem) * items.size()));
     if (sync_cap_ < 2 + items.size()) {   // shared by both schedules: the larger one's progress flags
         int err_word = 0;
-        if (d_sync) IDC_TRY_CUDA(cudaMemcpy(&err_word, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost));
+        if (d_sync) {
+            IDC_TRY_CUDA(cudaMemcpyAsync(&err_word, d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost, stream));
+            IDC_TRY_CUDA(cudaStreamSynchronize(stream));   // (also of sweeps still queued)
+        }
         cudaFree(d_sync);
         d_sync = nullptr;
         sync_cap_ = 0;
         IDC_TRY_CUDA(cudaMalloc(&d_sync, sizeof(int) * (2 + items.size())));
         sync_cap_ = 2 + items.size();
-        IDC_TRY_CUDA(cudaMemset(d_sync, 0, sizeof(int) * sync_cap_));
-        IDC_TRY_CUDA(cudaMemcpy(d_sync + 1, &err_word, sizeof(int), cudaMemcpyHostToDevice));   // kept until checked
+        IDC_TRY_CUDA(cudaMemsetAsync(d_sync, 0, sizeof(int) * sync_cap_, stream));
+        IDC_TRY(upload(d_sync + 1, &err_word, sizeof(int)));   // kept until checked
     }
 
     if (use_warp_kernel) {
@@ -1161,7 +1170,7 @@ Status Context::transport_residual_transpose(const double *z, double *y, double 
     if (!d_ones_) {
         std::vector<double> ones((size_t)nq, 1.0);
         IDC_TRY_CUDA(cudaMalloc(&d_ones_, sizeof(double) * nq));
-        IDC_TRY_CUDA(cudaMemcpy(d_ones_, ones.data(), sizeof(double) * nq, cudaMemcpyHostToDevice));
+        IDC_TRY(upload(d_ones_, ones.data(), sizeof(double) * nq));
     }
     IDC_TRY_CUDA(launch_pmv(dims(), 1.0, 0.0, d_ones_, z, zsum, stream));   // sum_q z_q
     IDC_TRY_CUDA(launch_lmv_transpose(dims(), 1.0, 0.0, d_sigma_t, d_xi, d_eta, d_w, z, y, stream, -1.0, d_sigma_s,

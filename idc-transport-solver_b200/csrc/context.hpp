@@ -41,6 +41,9 @@ public:
     // The stream waits for what the caller has queued on the legacy default stream (the library's streams are
     // non-blocking ones): every call that works on the caller's device arrays begins with this.
     Status after_caller();
+    // Host -> device on the context's own stream, complete on return: a set-up copy or clear on the default stream is not
+    // ordered before the kernels that use it (a pageable cudaMemcpy may return before the copy has ended, cudaMemset does).
+    Status upload(void *dst, const void *src, size_t bytes);
     // Sweep: out <- L^{-1} (src [+ scale * S phi_scatter]); phi (nullable) <- P out.  src may equal out.
     // src2 (modal kernel, forward): the source is src + src2_scale * src2 on interior cells, combined by the
     // sweep's aux warps (or, when its stages do not fit in shared memory, by a kernel into a scratch array)

@@ -163,7 +163,7 @@ Status Context::idc_integrate(double *psi, const double *Q, double dt, int64_t s
     while ((int)idc_phi_.size() < need_phi) {
         double *p = nullptr;
         IDC_TRY_CUDA(cudaMalloc(&p, sizeof(double) * nm));
-        IDC_TRY_CUDA(cudaMemset(p, 0, sizeof(double) * nm));
+        IDC_TRY_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * nm, stream));
         idc_phi_.push_back(p);
     }
     auto stage = [&](int l) { return idc_psi_[l]; };

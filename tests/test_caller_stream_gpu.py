@@ -83,13 +83,21 @@ def test_call_waits_for_the_default_stream(name):
         assert torch.equal(got[k], want[k]), k
 
 
-def test_set_sigma_waits_for_the_default_stream():
+@pytest.mark.parametrize("degree", [0, 1])
+def test_set_sigma_waits_for_the_default_stream(degree):
+    """Cross sections constant on each cell, and (degree 1) given by their Legendre moments."""
     import torch
     P = random_problem(24, 20, 1, 4, seed=3, dt=0.3)
-    with _context(P) as c:
-        want, got = P.source.copy(), P.source.copy()
+    if degree:
+        slopes = np.random.default_rng(2).uniform(-0.1, 0.1, (P.sigma_t.size, 4))
+        slopes[:, 0] = 1.0
+        P.sigma_t, P.sigma_s = P.sigma_t.reshape(-1, 1) * slopes, P.sigma_s.reshape(-1, 1) * slopes
+    want, got = P.source.copy(), P.source.copy()
+    with abi.SweepContext(P.nx, P.ny, P.p, P.ax, P.bx, P.ay, P.by, sigma_degree=degree) as c:
+        c.set_ordinates(P.xi, P.eta, P.w, P.quad)
+        c.set_sigma(P.sigma_t, P.sigma_s)
         c.sweep(want, P.dt)
-        st, ss = torch.from_numpy(P.sigma_t).cuda(), torch.from_numpy(P.sigma_s).cuda()
+        st, ss = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (P.sigma_t, P.sigma_s))
         a, b = torch.ones_like(st), torch.ones_like(ss)
         torch.cuda.synchronize()
         torch.cuda._sleep(20_000_000)
