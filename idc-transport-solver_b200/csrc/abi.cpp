@@ -395,24 +395,29 @@ int idc_gmres_solve(idc_ctx *ctx, double *source_inout, double dt, double abs_to
     idc::Context &c = ctx->impl;
     ABI_TRY_CUDA(cudaSetDevice(c.device));
     c.launches = 0;
-    // on the caller's device array in place (the source is read until the last sweep, which overwrites it): 256x256 Q2
-    // S16 without the three copies of psi 11.4 -> 10.7 ms
-    double *d_psi = source_inout;
+    // The source is read from the caller's device array, and psi goes there when the solve has succeeded: a solve that fails
+    // leaves the array as it came.
+    ABI_TRY(c.ensure_psi_buffers(1));
+    double *d_psi = c.psi_buf(0);
+    const double *d_src = source_inout;
     if (loc == IDC_LOC_HOST) {
-        ABI_TRY(c.ensure_psi_buffers(1));
-        d_psi = c.psi_buf(0);
         ABI_TRY_CUDA(cudaMemcpyAsync(d_psi, source_inout, sizeof(double) * c.psi_len(), cudaMemcpyHostToDevice, c.stream));
+        d_src = d_psi;
     } else {
         ABI_TRY(c.after_caller());
     }
     int64_t its = 0;
     double res = 0;
-    idc::Status st = c.gmres_peierls(d_psi, d_psi, dt, abs_tol, restart, max_its, precision, &its, &res);
+    idc::Status st = c.gmres_peierls(d_src, d_psi, dt, abs_tol, restart, max_its, precision, &its, &res);
     if (iters) *iters = its;
     if (final_resid) *final_resid = res;
     if (!st.good()) return fail(st);
     if (loc == IDC_LOC_HOST)
         ABI_TRY_CUDA(cudaMemcpyAsync(source_inout, d_psi, sizeof(double) * c.psi_len(), cudaMemcpyDeviceToHost, c.stream));
+    else if (c.ghost_mask())   // reflecting or periodic edges: the ghost values too
+        ABI_TRY_CUDA(cudaMemcpyAsync(source_inout, d_psi, sizeof(double) * c.psi_len(), cudaMemcpyDeviceToDevice, c.stream));
+    else
+        ABI_TRY_CUDA(idc::launch_copy_interior(c.dims(), d_psi, source_inout, c.stream));
     ABI_TRY_CUDA(cudaStreamSynchronize(c.stream));
     return IDC_OK;
     ABI_GUARD_END

@@ -336,15 +336,13 @@ __global__ void periodic_halos_kernel(GridDims g, double *__restrict__ psi) {
     }
 }
 
-// One thread per interior value: see launch_copy_interior.
+// The interior cells of a column are one run of ny cells: blocks (.., y) copy columns y, y + gridDim.y, ...
 __global__ void copy_interior_kernel(GridDims g, const double *__restrict__ src, double *__restrict__ dst) {
-    const size_t per = (size_t)g.nq * g.P * g.P;
-    const size_t total = (size_t)g.nx * g.ny * per;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const size_t cell = t / per, l = t % per;
-        const size_t i = 1 + cell / g.ny, j = 1 + cell % g.ny;
-        const size_t at = (i * (g.ny + 2) + j) * per + l;
-        dst[at] = src[at];
+    const size_t per = (size_t)g.nq * g.P * g.P, run = g.ny * per;
+    for (int i = 1 + blockIdx.y; i <= g.nx; i += gridDim.y) {
+        const size_t at = ((size_t)i * (g.ny + 2) + 1) * per;
+        for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < run; t += (size_t)gridDim.x * blockDim.x)
+            dst[at + t] = src[at + t];
     }
 }
 
@@ -999,8 +997,9 @@ cudaError_t launch_periodic_halos(const GridDims &g, double *psi, cudaStream_t s
 }
 
 cudaError_t launch_copy_interior(const GridDims &g, const double *src, double *dst, cudaStream_t s) {
-    const size_t total = (size_t)g.nx * g.ny * g.nq * g.P * g.P;
-    copy_interior_kernel<<<blocks_for(total), kThreads, 0, s>>>(g, src, dst);
+    const size_t run = (size_t)g.ny * g.nq * g.P * g.P, want = (run + kThreads - 1) / kThreads;
+    const unsigned columns = (unsigned)(g.nx < 148 * 16 ? g.nx : 148 * 16), most = 148 * 16 / columns + 1;
+    copy_interior_kernel<<<dim3(want < most ? (unsigned)want : most, columns), kThreads, 0, s>>>(g, src, dst);
     return cudaGetLastError();
 }
 

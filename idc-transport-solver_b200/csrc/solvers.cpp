@@ -272,11 +272,9 @@ Status Context::gmres_peierls_boundary(const double *src, double *psi_out, doubl
                   ng));
     if (src != psi_out)
         IDC_TRY_CUDA(cudaMemcpyAsync(psi_out, src, sizeof(double) * psi_len(), cudaMemcpyDeviceToDevice, stream));
-    if (converged || src != psi_out) {   // in place the source outlives a solve that failed
-        IDC_TRY(reflect_ghosts(psi_out, x + np, false));
-        IDC_TRY(smv(1.0, 1.0, x, psi_out));
-        IDC_TRY(boundary_sweep(psi_out, dt, nullptr, precision));
-    }
+    IDC_TRY(reflect_ghosts(psi_out, x + np, false));
+    IDC_TRY(smv(1.0, 1.0, x, psi_out));
+    IDC_TRY(boundary_sweep(psi_out, dt, nullptr, precision));
     IDC_TRY(check_device_error());
     if (resid_out) *resid_out = resid;
     if (!converged)
@@ -305,8 +303,8 @@ Status Context::gmres_peierls(const double *src, double *psi_out, double dt, dou
         IDC_TRY_CUDA(cudaMemcpyAsync(x, phi_guess, sizeof(double) * phi_len(), cudaMemcpyDeviceToDevice, stream));
     IDC_TRY(gmres(op, b, x, abs_tol, restart, max_its, iters_out, &resid, &converged, precond_kind == 1 ? 1 : 0, 0,
                   phi_guess != nullptr));
-    // psi = L^{-1} (S phi + Q)  (PETScPeierlsSolver.cpp:504-505); in place the source outlives a solve that failed
-    if (converged || src != psi_out) IDC_TRY(sweep(src, psi_out, dt, nullptr, precision, x, 1.0));
+    // psi = L^{-1} (S phi + Q)  (PETScPeierlsSolver.cpp:504-505)
+    IDC_TRY(sweep(src, psi_out, dt, nullptr, precision, x, 1.0));
     IDC_TRY(check_device_error());
     if (resid_out) *resid_out = resid;
     if (!converged)
@@ -358,7 +356,7 @@ Status Context::gmres_peierls_ir(const double *src, double *psi_out, double dt, 
         IDC_TRY_CUDA(launch_axpby(-1.0, ax, 1.0, r, n, stream));
         launches += 3;
     }
-    if (converged || src != psi_out) IDC_TRY(sweep(src, psi_out, dt, nullptr, IDC_PREC_FP64, x, 1.0));
+    IDC_TRY(sweep(src, psi_out, dt, nullptr, IDC_PREC_FP64, x, 1.0));
     IDC_TRY(check_device_error());
     if (iters_out) *iters_out = total;
     if (resid_out) *resid_out = resid;

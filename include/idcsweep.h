@@ -186,7 +186,8 @@ int idc_sweep_noalloc(const idc_problem_desc *desc, int64_t nq, const double *xi
  * iterations; each correction adds one FP64 residual sweep).  Replaces
  * PETScPeierlsSolver::Solve with IPLS (linear_solvers/Abstract/ImplicitSolver/PETScPeierlsSolver.cpp:423-572);
  * PETSc's LGMRES augmentation is not reproduced (same fixed point, different iteration counts).  Returns
- * IDC_ERR_NOT_CONVERGED after max_its iterations, as the reference throws. */
+ * IDC_ERR_NOT_CONVERGED after max_its iterations, as the reference throws.  A solve that fails leaves
+ * source_inout as it came. */
 int idc_gmres_solve(idc_ctx *ctx, double *source_inout, double dt, double abs_tol, int32_t restart, int64_t max_its,
                     int precision, int loc, int64_t *iters, double *final_resid);
 

@@ -50,8 +50,8 @@ def test_sweep_wait_gives_up_and_context_recovers(restatement):
 
 
 def test_gmres_dsa_timeout_then_bitwise_recovery():
-    """A GMRES + DSA solve whose sweeps and DSA grid barriers give up, then the same solve with the default
-    bound, bitwise equal to the solve on a context that never failed."""
+    """A GMRES + DSA solve whose sweeps give up, then the same solve with the default bound, bitwise equal to the
+    solve on a context that never failed."""
     P = random_problem(48, 72, 1, 8, seed=78)
     with _ctx(P) as c:
         c.set_preconditioner(abi.PRECOND_DSA, 10)
@@ -67,3 +67,28 @@ def test_gmres_dsa_timeout_then_bitwise_recovery():
         its, _ = c.gmres_solve(psi, P.dt, abs_tol=1e-10, restart=20, max_its=500)
     assert its == its_ref
     assert np.array_equal(psi, src)
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_FP32_IR])
+def test_gmres_on_a_device_array_keeps_the_source_when_the_last_sweep_gives_up(precision):
+    """The solve converges at once (any residual is small enough) and only its last sweep, which forms psi, gives up: the
+    caller's array still holds the source, and the same solve with the default bound succeeds on it."""
+    import torch
+    P = random_problem(64, 96, 2, 8, seed=79, dt=0.1)
+    with _ctx(P) as c:
+        def shorten(ptr, n):   # called after every moment sum: the right-hand side's is the only one
+            c.set_spin_limit(limit[0])
+            return 0
+
+        c.set_allreduce(shorten)
+        psi = torch.from_numpy(P.source).cuda()
+        torch.cuda.synchronize()
+        limit = [2]
+        _expect_timeout(lambda: c.gmres_solve(psi.data_ptr(), P.dt, abs_tol=1e300, precision=precision, loc=abi.LOC_DEVICE))
+        assert np.array_equal(psi.cpu().numpy(), P.source)
+        limit = [0]
+        c.set_spin_limit(0)
+        c.gmres_solve(psi.data_ptr(), P.dt, abs_tol=1e300, precision=precision, loc=abi.LOC_DEVICE)
+        want = P.source.copy()
+        c.gmres_solve(want, P.dt, abs_tol=1e300, precision=precision)
+    assert np.array_equal(psi.cpu().numpy(), want)
