@@ -1,16 +1,20 @@
 """Edges of the lane kernel's tiles and of the solvers' one-launch kernels, against the CPU restatement.
 
-* Sweeps: row counts around whole thread blocks (3, 4 or 7 warps of 32/seg rows) and one row block, columns around the
-  copy and trace rings, quadrants with unequal, odd and zero ordinate counts (row segments that start and end off a
-  16-byte boundary), arrays off a 16- and a 32-byte boundary.
+* Sweeps: few chains (thread blocks of 3 warps of 32/seg rows), rows around one row block, columns around the copy and
+  trace rings, quadrants with unequal, odd and zero ordinate counts (row segments that start and end off a 16-byte
+  boundary), arrays off a 16- and a 32-byte boundary.
+* Sweeps of every instance (plain, FP32, transposed, moments-only, two sources) with as many chains as take thread blocks
+  of 4 and of 7 warps, rows around whole blocks, and more items than blocks in flight, so that blocks take several.
 * DSA: grids around the cluster shapes (512 cells per block, 1 to 16 blocks, 1 to 8 cells per thread) and beyond the
-  largest; the preconditioned solve must converge in fewer iterations to the same flux.
+  largest; the preconditioned solve must converge in fewer iterations to the same flux (a single application is compared
+  in test_solver_kernels_gpu.py).
 * Batches: the moments-only sweeps of uneven members, one of them converged long before the others.
 """
 import numpy as np
 import pytest
 
 from conftest import rel_err, to_oracle
+from idc_ref import idc_steps
 from idcsweep import abi
 from idcsweep.problems import Problem, random_problem
 
@@ -69,6 +73,79 @@ def test_tile_edges(restatement, p, seg, nx, ny, counts, offset):
         assert np.all(got == 7.0)   # no store outside the interior cells
         c.sweep(src.data_ptr(), P.dt, phi.data_ptr(), loc=abi.LOC_DEVICE)   # in place
         assert rel_err(src.cpu().numpy().reshape(P.psi_shape())[1:-1, 1:-1], ref[1:-1, 1:-1]) < TOL64
+
+
+def _warps(p, seg, counts, ny):
+    """The rule for the warps of a thread block (3, 4 or 7), and the launch's items."""
+    widest = -(-max(counts) // -(-max(counts) // seg))
+    chains = sum(-(-n // widest) for n in counts)
+    items = {w: chains * -(-ny // (w * 32 // seg)) for w in (3, 4, 7)}
+    w = 3 if items[3] <= 148 else 4 if items[4] <= (148 * 4 // 3 if p == 2 else 148) else 7
+    return w, items[w]
+
+
+# segment width, columns, rows, ordinates per quadrant: 128 = 4 blocks of 4 warps, 280 = 5 of 7; two chunks and more
+SHAPES = [(4, 17, 127, (36, 35, 33, 34)), (4, 15, 128, (36, 35, 33, 34)), (4, 16, 129, (36, 35, 33, 34)),
+          (4, 16, 279, (36, 35, 33, 34)), (4, 7, 280, (36, 35, 33, 34)), (4, 17, 281, (36, 35, 33, 34)),
+          (16, 16, 183, (33, 31, 32, 17)), (8, 15, 533, (9, 7, 8, 10))]
+
+
+def test_shapes_reach_what_they_claim():
+    got = {(p, *_warps(p, seg, counts, ny)) for p in (0, 1, 2) for seg, nx, ny, counts in SHAPES}
+    for p in (0, 1, 2):
+        assert any(q == p and w == 4 for q, w, n in got)
+        assert any(q == p and w == 7 and n > 148 for q, w, n in got)
+
+
+@pytest.mark.parametrize("p", [0, 1, 2])
+@pytest.mark.parametrize("seg,nx,ny,counts", SHAPES)
+def test_larger_thread_blocks(restatement, p, seg, nx, ny, counts):
+    import torch
+    P = _uneven(nx, ny, p, counts, seed=nx + ny + p, dt=0.3)
+    O = to_oracle(P)
+    core = np.s_[1:-1, 1:-1]
+    with _ctx(P) as c:
+        c.set_tile_shape(seg, 0)
+        src, out = _device(P.source, 1), _device(np.zeros(P.source.shape), 3)
+        phi = torch.zeros(P.phi_shape(), dtype=torch.float64, device="cuda")
+
+        def psi():
+            return out.cpu().numpy().reshape(P.psi_shape())[core]
+
+        ref = restatement.sweep(O, P.source, P.dt).reshape(P.psi_shape())
+        ref_phi = restatement.pmv(O, ref).reshape(P.phi_shape())
+        # FP32: 2^-24 times the operations along the longest path, about 10 a cell
+        for prec, tol in ((abi.PREC_FP64, TOL64), (abi.PREC_FP32, 2.0 ** -24 * 10 * (nx + ny))):
+            c.sweep_out(src.data_ptr(), out.data_ptr(), P.dt, phi.data_ptr(), prec, abi.LOC_DEVICE)
+            assert rel_err(psi(), ref[core]) < tol, prec
+            assert rel_err(phi.cpu().numpy(), ref_phi) < tol, prec
+
+        ref = restatement.sweep_adjoint(O, P.source, P.dt).reshape(P.psi_shape())
+        c.sweep_adjoint(src.data_ptr(), out.data_ptr(), P.dt, phi.data_ptr(), loc=abi.LOC_DEVICE)
+        assert rel_err(psi(), ref[core]) < TOL64
+        assert rel_err(phi.cpu().numpy()[core], ref[core].sum(axis=2)) < TOL64
+
+        x = np.random.default_rng(ny).uniform(-0.5, 1.0, P.phi_shape())
+        scattered = np.zeros(P.psi_shape())
+        scattered[core] = restatement.smv(O, x, np.zeros(P.psi_shape())).reshape(P.psi_shape())[core]
+        ref_phi = restatement.pmv(O, restatement.sweep(O, scattered, P.dt)).reshape(P.phi_shape())
+        dx = torch.from_numpy(x).cuda()
+        c.sweep_fused(None, None, P.dt, dx.data_ptr(), 1.0, phi.data_ptr())
+        assert rel_err(phi.cpu().numpy(), ref_phi) < TOL64
+
+
+@pytest.mark.parametrize("p,seg,nx,ny,counts", [(0, 4, 16, 129, (36, 35, 33, 34)), (1, 8, 15, 533, (9, 7, 8, 10)),
+                                                (1, 4, 17, 127, (36, 35, 33, 34)), (2, 16, 6, 183, (33, 31, 32, 17))])
+def test_larger_thread_blocks_two_sources(restatement, p, seg, nx, ny, counts):
+    """One explicit IDC step, whose correction sweeps have two sources, each with its own row segments' alignment."""
+    P = _uneven(nx, ny, p, counts, seed=nx + ny + p, dt=0.05)
+    P.source[0], P.source[-1], P.source[:, 0], P.source[:, -1] = 0.0, 0.0, 0.0, 0.0
+    psi = np.zeros(P.psi_shape())
+    want = idc_steps(restatement, to_oracle(P), psi, P.source, P.dt, 1, M=3, K=1, scattering="explicit")
+    with _ctx(P) as c:
+        c.set_tile_shape(seg, 0)
+        c.idc_integrate(psi, P.source, P.dt, 1, 3, 1, abi.SCATTER_EXPLICIT, use_graph=False)
+    assert rel_err(psi[1:-1, 1:-1], want[1:-1, 1:-1]) < TOL64
 
 
 @pytest.mark.parametrize("nx,ny", [(1, 1), (1, 513), (64, 16), (91, 90), (92, 90), (129, 127), (182, 181), (256, 256),
