@@ -353,7 +353,8 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
     for (Group *g : used) IDC_TRY(launch_group(*g, srcs, outs, phi_sc, scale, phis, dt, active, peierls));
     IDC_TRY_CUDA(cudaEventRecord(c0.ev1, c0.stream));
     IDC_TRY_CUDA(cudaStreamSynchronize(c0.stream));
-    for (Group *gp : used) {
+    bool gave_up = false;
+    for (Group *gp : used) {   // every group that failed is re-armed: the next call starts clean
         Group &g = *gp;
         int err = 0;
         IDC_TRY_CUDA(cudaMemcpy(&err, g.d_sync + 1, sizeof(int), cudaMemcpyDeviceToHost));
@@ -363,9 +364,10 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
                 IDC_TRY_CUDA(launch_fill_u64(reinterpret_cast<unsigned long long *>(g.trace[m]), g.trace_len[m],
                                              kTraceSentinel, c0.stream));
             IDC_TRY_CUDA(cudaStreamSynchronize(c0.stream));
-            return bad(IDC_ERR_TIMEOUT, "a device-side wait gave up in a batched sweep");
+            gave_up = true;
         }
     }
+    if (gave_up) return bad(IDC_ERR_TIMEOUT, "a device-side wait gave up in a batched sweep");
     float ms = 0.f;
     IDC_TRY_CUDA(cudaEventElapsedTime(&ms, c0.ev0, c0.ev1));
     last_ms = ms;

@@ -92,3 +92,25 @@ def test_gmres_on_a_device_array_keeps_the_source_when_the_last_sweep_gives_up(p
         want = P.source.copy()
         c.gmres_solve(want, P.dt, abs_tol=1e300, precision=precision)
     assert np.array_equal(psi.cpu().numpy(), want)
+
+
+def test_batched_sweep_gives_up_and_the_next_one_is_right(restatement):
+    """Members of two degrees, a launch each, both of which give up: one failed call, and the next is right."""
+    import torch
+    probs = [random_problem(40, 96, 1, 8, seed=81, dt=0.1), random_problem(40, 96, 2, 8, seed=82, dt=0.1)]
+    ctxs = [_ctx(P) for P in probs]
+    srcs = [torch.from_numpy(P.source).cuda() for P in probs]
+    outs = [torch.zeros_like(s) for s in srcs]
+    with abi.Batch() as b:
+        for c in ctxs:
+            b.add(c)
+            c.set_spin_limit(2)
+        args = [s.data_ptr() for s in srcs], [o.data_ptr() for o in outs], None, 0.1
+        _expect_timeout(lambda: b.sweep(*args))
+        for c in ctxs:
+            c.set_spin_limit(0)
+        b.sweep(*args)
+    for P, c, out in zip(probs, ctxs, outs):
+        ref = restatement.sweep(to_oracle(P), P.source, P.dt).reshape(P.psi_shape())
+        assert rel_err(out.cpu().numpy()[1:-1, 1:-1], ref[1:-1, 1:-1]) < TOL64
+        c.close()
