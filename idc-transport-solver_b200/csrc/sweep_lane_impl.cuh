@@ -226,9 +226,8 @@ __device__ __forceinline__ int wait_for_credit(uint32_t consumed, int column, in
                                                unsigned sleep_ns) {
     for (long long polls = 0;;) {
         for (int k = 0; k < kReadsPerPoll; ++k) {
-            int c = 0;
-            if (lane == 0) c = ld_consumed(consumed);
-            c = __shfl_sync(kFullMask, c, 0);
+            // (every lane acquires the count itself: its writes are ordered after the reader's re-arming)
+            const int c = (int)__reduce_min_sync(kFullMask, (unsigned)ld_consumed(consumed));
             if (column < c + kRing) return c + kRing;
             __nanosleep(sleep_ns);
         }
