@@ -310,8 +310,8 @@ def extra_idc(abi, torch, dev, steps=10):
         psi = torch.zeros(P.psi_shape(), dtype=torch.float64, device=f"cuda:{dev}")
         src = torch.from_numpy(P.source).to(f"cuda:{dev}")
         for name, prec in (("fp64", abi.PREC_FP64), ("fp32_refined", abi.PREC_FP32_REFINED)):
-            # the autotuner times plain sweeps; the library's default picks the IMEX sweeps' kernel by grid size
-            # (the lane kernel, narrow segments at Q1), so FP64 keeps it
+            # the autotuner times plain sweeps; the IMEX sweeps' default in FP64 is the lane kernel with narrow segments
+            # at Q1, which is kept
             if prec == abi.PREC_FP64:
                 c.set_tile_shape(0, 0)
                 out.setdefault("tile_shape", {})[name] = "default (IMEX at Q1: lane, seg 4)"

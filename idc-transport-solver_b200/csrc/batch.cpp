@@ -326,8 +326,8 @@ Status Batch::sweep(const double *const *srcs, double *const *outs, const double
     for (auto &g : groups) {
         Group *u = &g;
         if (peierls && g.wn == 0 && !tuned.count(std::make_pair(g.P, precision))) {
-            // moments-only sweeps have their own default width, as a single problem's (256x256 Q2 S8: 247 us against
-            // 318 with the full sweep's 16-wide segments)
+            // moments-only sweeps have their own default width, as a single problem's (256x256 Q2 S8: 234 us against
+            // 288 with the full sweep's 16-wide segments)
             int qmax = 0;
             for (int m : g.members) qmax = std::max(qmax, qmax_of(*members[m]));
             const int seg = narrow_seg(qmax, true);

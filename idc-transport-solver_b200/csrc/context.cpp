@@ -695,8 +695,9 @@ Status Context::build_schedule(int precision) {
                            modal_like, &G, &seg, &wn);
         if (active == kLane && sched_variant_ != 1 && user_G == 0 && user_R == 0 && P == 3) {
             // full sweeps at DG degree 2: 16-wide segments (fewer partial moments, and their sums from shared memory
-            // instead of shuffles); B200, 256x256 S16: 671 us, 722 with 8, 697 with 4; 192x160 S12 359, 379 with 4.  At
-            // degrees 0 and 1, and for the moments-only sweeps, the narrowest: 512x512 Q1 S12 753, 776 with 8
+            // instead of shuffles); B200, sweep kernel: 256x256 S16 600 us, 673 with 8, 660 with 4; 192x160 S12 316, 324,
+            // 359; 128x128 S8 199, 226, 253.  At degrees 0 and 1, and for the moments-only sweeps, the narrowest:
+            // 512x512 Q1 S12 687 us with 4, 719 with 8, 795 with 16; moments-only 256x256 Q2 S16 298, 369, 364
             seg = 16;
             const int nch = (qmax + seg - 1) / seg;
             G = (qmax + nch - 1) / nch;

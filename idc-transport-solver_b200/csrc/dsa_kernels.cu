@@ -9,11 +9,12 @@
 // is the classic DSA correction: for the flat mode of an infinite medium, (I - P L^{-1} S)^{-1} =
 // 1 + sigma_s / sigma_a exactly.  Faces use the harmonic mean of the two cells' D (uniform grid); a
 // boundary face is a Marshak vacuum condition, flux = u_b / 2 with D (u - u_b) / (h/2) = u_b / 2.
-// The right-hand side and all Jacobi-PCG steps run in one cooperative kernel (every block resident), in
-// the Chronopoulos-Gear form of CG with one global reduction and one grid barrier per step; each block adds
-// the per-block partial sums in the same fixed order, so the step lengths are identical on every block and
-// the result is bitwise reproducible.  The barrier waits are bounded: on expiry the device error word is
-// set and every block leaves.
+// The right-hand side and all Jacobi-PCG steps run in one kernel, in the Chronopoulos-Gear form of CG with one
+// global reduction per step: a thread-block cluster per problem up to kClusterCells cells, a cooperative kernel
+// (every block resident) beyond.  Each block adds the partial sums in the same fixed order, so the step lengths
+// are identical on every block and the result is bitwise reproducible.  The cooperative kernel's barrier waits are
+// bounded: on expiry the device error word is set and every block leaves.  The cluster's barrier is the hardware's,
+// whose blocks run together by construction and wait for nothing else.
 #include "device_sync.cuh"
 #include "idc_internal.hpp"
 
@@ -90,9 +91,6 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // Grid barrier number e (0, 1, ...) of a cooperative launch on an arrival counter that is zero when the

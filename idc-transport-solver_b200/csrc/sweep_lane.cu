@@ -199,9 +199,13 @@ bool sweep_lane_supports(int P, int precision, int seg) {
 // latency of an iteration, and two warps on one SM sub-partition slow each other: 3 warps and the helper (one warp per
 // sub-partition) while every block then has an SM of its own, else 4 likewise; large ones by the warps in flight and the
 // handoffs through L2 between blocks: 7 and the helper.  At DG degree 2, whose iterations keep a sub-partition busier, 4
-// up to 4/3 blocks per SM.  B200, sweep kernel in us with 3 / 4 / 7 warps: 64x64 Q1 S8 66.5 / - / 73.7, 128x128 Q1 S16
-// 159 / 137 / 153, 192x160 Q2 S12 381 / 359 / 378, 256x256 Q1 S12 316 / 323 / 307, 256x256 Q2 S16 691 / - / 671; its
-// moments-only sweep 370 / - / 324.
+// up to 4/3 blocks per SM.  B200, sweep kernel in us with 3 / 4 / 7 warps (in brackets the blocks with 4):
+//   degrees 0 and 1: 64x64 Q1 S8 65.6 / 67.6 / 71.7 (24), 256x128 Q1 S12 185 / 191 / 211 (96), 128x128 Q1 S16 150 / 130 / 141
+//   (144), 256x256 Q1 S12 295 / 303 / 283 (192), 300x200 Q0 S16 234 / 218 / 204 (252), 512x512 Q1 S12 766 / 692 / 688 (384);
+//   degree 2: 131x197 S10 267 / 270 / 322 (100), 192x128 S12 315 / 260 / 315 (128), 192x160 S12 352 / 315 / 345 (160),
+//   128x128 S16 260 / 227 / 249 (192), 192x200 S12 404 / 351 / 383 (200), 128x144 S16 281 / 242 / 262 (216), 256x256 S16
+//   633 / 633 / 600 (384): 4 warps stay ahead a little beyond the line;
+//   moments-only: 64x64 Q1 S8 51.2 / 51.2 / 55.3, 128x128 Q2 S16 154 / 124 / 146, 256x256 Q2 S16 346 / 307 / 297.
 int sweep_lane_warps(int P, int seg, bool src2, int num_sms, const std::function<int64_t(int)> &row_blocks) {
     int w = row_blocks(3) <= num_sms                              ? 3
             : row_blocks(4) <= (P == 3 ? num_sms * 4 / 3 : num_sms) ? 4

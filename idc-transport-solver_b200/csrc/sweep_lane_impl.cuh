@@ -29,13 +29,13 @@
 // sizes, issue slots the large ones.  Measured on B200 (sweep kernel, before -> after each):
 //   * handoff through shared memory, L2 only between blocks and there by the helper: when every warp read the trace of
 //     the row above from L2 itself, no iteration could be shorter than an L2 load (0.56 us at degree 0, where it is 0.2
-//     us of work).  With the rest below, 300x200 Q0 S16 349 -> 202 us, 64x64 Q1 S8 85 -> 66 us, 512x512 Q1 S12 932 -> 753
-//     us; 256x256 Q2 S16 (684 -> 671 us) is bound by issue: 648 warp instructions per iteration, 215 of them FP64, with
-//     255 registers and so two warps per sub-partition.
+//     us of work).  With the rest below, 300x200 Q0 S16 349 -> 204 us, 64x64 Q1 S8 85 -> 66 us, 512x512 Q1 S12 932 -> 688
+//     us; 256x256 Q2 S16 (684 -> 600 us) is bound by issue and latency: 633 warp instructions per iteration, 217 of them
+//     FP64, with 253 registers and so two warps per sub-partition.
 //   * psi stores: bulk copies through shared memory (proxy fence, commit, wait) cost 0.25 us an iteration at degree 1;
 //     a lane's own 32-byte store 0.001 (2048x4 Q1 S8, one row block: 1342 -> 832 us).  Degree 2: 16-byte chunks.
 //   * the moments-only sweeps' inputs (modal source and sigma_t) as one record per cell copied once per row, where every
-//     lane had copied its own: 256x256 Q2 S16 566 -> 324 us with the above, 128x128 Q1 S8 117 -> 93 us.
+//     lane had copied its own: 256x256 Q2 S16 566 -> 297 us with the above, 128x128 Q1 S8 117 -> 97 us.
 //   * the backward transform in its own iteration instead of beside the next one's chain: 38 fewer live registers, no
 //     spills at degree 2 (2048x2 Q2 S16, one row block: 1766 -> 1460 us).
 //
@@ -138,7 +138,7 @@ __device__ __forceinline__ void segment_sums(T (&v)[N], int o, int *lo, int *hi)
 }
 
 // Global accesses under a predicate instead of a branch, so that the loop body stays one basic block and
-// the scheduler can interleave the three cells' work.  An access whose predicate is false is not made.
+// the scheduler can interleave the parts of an iteration.  An access whose predicate is false is not made.
 __device__ __forceinline__ void st_f64_if(double *p, double v, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.global.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
                  "r"((int)pred));

@@ -37,7 +37,8 @@ enum {
     IDC_ERR_ARG = 1,            /* invalid argument (null pointer, bad size, unsorted ordinates, ...)   */
     IDC_ERR_UNSUPPORTED = 2,    /* valid for the reference but not implemented here (e.g. p > 2)        */
     IDC_ERR_CUDA = 3,           /* a CUDA runtime call failed; idc_last_error_message() has the text     */
-    IDC_ERR_TIMEOUT = 4,        /* a device-side wait gave up (bounded spin); results are not valid      */
+    IDC_ERR_TIMEOUT = 4,        /* a device-side wait gave up (bounded spin); results are not valid, and  */
+                                /* an array that the call works on in place is lost unless it says not   */
     IDC_ERR_NOT_CONVERGED = 5,  /* an iterative solve stopped at its iteration limit                     */
     IDC_ERR_STATE = 6,          /* call order violated (e.g. sweep before idc_set_ordinates)             */
     IDC_ERR_NOMEM = 7           /* device allocation failed                                              */
@@ -86,7 +87,8 @@ int idc_set_ordinates(idc_ctx *ctx, int64_t nq, const double *xi, const double *
 /* Installs sigma_t and sigma_s on the halo-padded cell grid (loc as above): one value per cell when
  * sigma_degree = 0, or, when sigma_degree = dg_degree (high-order cross sections), the (p+1)^2 Legendre
  * moments of each cell, [cell][u][v] as the CrossSection's DensityFunction array holds them.  sigma_s may
- * be NULL (treated as zero).  These are the CrossSection arguments of SweepOperator::Apply and
+ * be NULL (treated as zero).  Values are finite, but that at DG degree 0 sigma_t may be infinite (a black cell: psi
+ * is zero there).  These are the CrossSection arguments of SweepOperator::Apply and
  * ImplicitSolver::Solve.  High-order cross sections enter as the reference's tensor branches do: the cell
  * matrix of CalcA (linear_solvers/RKDG/SweepCellSolve/SweepLinearSolveSpec.cpp:298-318), Smv and Lmv
  * (operators/RKDG/TransportOperator.cpp:367-386, :1335-1359), with the tensor of Legendre triple products of
@@ -244,7 +246,7 @@ int idc_sweep_fused(idc_ctx *ctx, const double *source, double *result, double d
 int idc_set_tile_shape(idc_ctx *ctx, int32_t seg, int32_t warps);
 
 /* Autotuner: times every tile shape of both kernels on this context's problem with `source` (device psi
- * array; plain sweeps: the IMEX sweeps of idc_idc_integrate may prefer another shape) and keeps the fastest (reported in *seg, *warps; warps = 0: the lane kernel). */
+ * array; plain sweeps are what is timed) and keeps the fastest (reported in *seg, *warps; warps = 0: the lane kernel). */
 int idc_autotune(idc_ctx *ctx, const double *source, double dt, int precision, int32_t *seg, int32_t *warps);
 
 /* A batch of independent problems (contexts on one GPU) swept together: one persistent launch per DG
@@ -271,7 +273,7 @@ int idc_batch_get_shape(idc_batch *b, int dg_degree, int precision, int32_t *seg
  * one synchronisation; converged members drop out of the launches.  psi_inout: host array of device
  * pointers, one per member in order (Q on entry, psi on return); iters and final_resids (nullable): host
  * arrays with one entry per member.  FP64 or FP32_REFINED sweeps.  IDC_ERR_NOT_CONVERGED if a member
- * stopped at max_its.  The batched form of PETScPeierlsSolver::Solve (linear_solvers/Abstract/
+ * stopped at max_its.  Works in place: after IDC_ERR_TIMEOUT the members' sources are lost.  The batched form of PETScPeierlsSolver::Solve (linear_solvers/Abstract/
  * ImplicitSolver/PETScPeierlsSolver.cpp:423-572) for many independent problems; the reference solves one. */
 int idc_batch_gmres_solve(idc_batch *b, double *const *psi_inout, double dt, double abs_tol, int32_t restart,
                           int64_t max_its, int precision, int64_t *iters, double *final_resids);
@@ -370,8 +372,9 @@ const char *idc_strerror(int status);
 /* Text of the most recent error on this thread (static per-thread storage). */
 const char *idc_last_error_message(void);
 
-/* Bound of every device-side wait of the context's kernels (a wait on another warp's or thread block's
- * progress, polled or blocking in the barrier unit): after `polls` polls the wait gives up, the kernel
+/* Bound of every device-side wait of the context's kernels on another warp's or thread block's progress, polled or
+ * blocking in the barrier unit (but for the hardware barrier of a thread-block cluster, whose blocks run together by
+ * construction: the DSA preconditioner up to 65536 cells): after `polls` polls the wait gives up, the kernel
  * records the failure in the context's device error word, every warp leaves, and the call returns
  * IDC_ERR_TIMEOUT after re-arming the context's trace buffers, so the next call starts clean.  polls <= 0
  * restores the default (2^22 polls, seconds of waiting; a sweep's waits normally end within microseconds).
