@@ -164,7 +164,7 @@ Status Batch::build_group(Group &g, int precision) {
     IDC_TRY_CUDA(cudaMalloc(&g.d_items, sizeof(SweepItem) * items.size()));
     IDC_TRY(c0.upload(g.d_items, items.data(), sizeof(SweepItem) * items.size()));
     IDC_TRY_CUDA(cudaMalloc(&g.d_sync, sizeof(int) * 2));
-    IDC_TRY_CUDA(cudaMemsetAsync(g.d_sync, 0, sizeof(int) * 2, c0.stream));
+    IDC_TRY_CUDA(cudaMemsetAsync(g.d_sync, 0, sizeof(int) * 2, stream()));
     IDC_TRY_CUDA(cudaMalloc(&g.d_table, sizeof(SweepArgs) * g.members.size()));
     IDC_TRY_CUDA(cudaMallocHost(&g.h_table, sizeof(SweepArgs) * g.members.size()));
     IDC_TRY_CUDA(cudaEventCreateWithFlags(&g.upload_done, cudaEventDisableTiming));

@@ -598,8 +598,9 @@ Status Context::ensure_phi_buffers(int count) {
     while ((int)phi_bufs_.size() < count) {
         double *p = nullptr;
         IDC_TRY_CUDA(cudaMalloc(&p, sizeof(double) * phi_len()));
-        IDC_TRY_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * phi_len(), stream));
         phi_bufs_.push_back(p);
+        IDC_TRY_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * phi_len(), stream));
+        IDC_TRY_CUDA(cudaStreamSynchronize(stream));   // (a batch uses it on another member's stream)
     }
     return Status::ok();
 }
