@@ -157,3 +157,21 @@ def test_solves_are_bitwise_reproducible(dsa):
     (a0, b0, *r0), (a1, b1, *r1) = outs
     assert np.array_equal(a0, a1) and np.array_equal(b0, b1)
     assert r0 == r1
+
+
+@pytest.mark.parametrize("edges", ["vacuum", "reflecting", "periodic"])
+def test_gmres_on_a_device_array_is_the_host_call(edges):
+    """psi comes back into the caller's device array cell for cell as into a host array: interior cells, and the ghost
+    values that reflecting and periodic edges leave."""
+    import torch
+    P = random_problem(11, 7, 1, 4, seed=17, dt=0.4)
+    with context_for(P) as ctx:
+        if edges == "reflecting":
+            ctx.set_reflecting(abi.EDGE_X_MIN | abi.EDGE_Y_MAX)
+        elif edges == "periodic":
+            ctx.set_periodic(True)
+        host = P.source.copy()
+        dev = torch.from_numpy(P.source).cuda()
+        assert ctx.gmres_solve(host, P.dt, 1e-10) == ctx.gmres_solve(dev.data_ptr(), P.dt, 1e-10, loc=abi.LOC_DEVICE)
+    assert np.array_equal(dev.cpu().numpy(), host)
+    assert np.array_equal(host[0], P.source[0]) == (edges == "vacuum")
